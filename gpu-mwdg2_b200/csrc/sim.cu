@@ -910,6 +910,7 @@ template <typename T> mwdg2_status Sim<T>::collect_step()
     last_cnt_[0] = (int64_t)sc_host_->enc;
     last_cnt_[1] = (int64_t)sc_host_->enc2;
     last_cnt_[2] = (int64_t)sc_host_->dec;
+    for (int l = mw::kBandMaxLevel + 1; l < L_ && l < 16; ++l) last_cnt_[2] += sc_host_->sig_level[l];
     last_cnt_[3] = sc_host_->n_leaves;
     last_cnt_[4] = n_det_ - 3;
     last_cnt_[5] = launches_;
