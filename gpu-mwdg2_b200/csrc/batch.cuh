@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 4) k_members_stage_w
 }
 
 template <typename T, int STAGE>
-__global__ void __launch_bounds__(kSolverThreads, sizeof(T) == 4 ? 5 : 2) k_members_stage_list(const __grid_constant__ MemberTable<T> tab,
+__global__ void __launch_bounds__(kSolverThreads, kStageBlocks<T>) k_members_stage_list(const __grid_constant__ MemberTable<T> tab,
                                                                                               const uint8_t* on,
                                                                                               const int32_t* first,
                                                                                               int n)

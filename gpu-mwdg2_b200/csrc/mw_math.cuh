@@ -221,14 +221,17 @@ template <typename T> MW_HD V3<T> phys_flux_x(const V3<T>& U, T tol_h, T g)
     if (U.h < tol_h) return {T(0), T(0), T(0)};
     return {U.qx, U.qx * U.qx / U.h + g * U.h * U.h / T(2.0), U.qx * U.qy / U.h};
 }
-template <typename T> MW_HD V3<T> phys_flux_y(const V3<T>& U, T tol_h, T g)
-{
-    if (U.h < tol_h) return {T(0), T(0), T(0)};
-    return {U.qy, U.qx * U.qy / U.h, U.qy * U.qy / U.h + g * U.h * U.h / T(2.0)};
-}
 
 // operators/flux_HLL.cuh:9-111
-template <typename T> MW_HD V3<T> flux_hll_x(const V3<T>& Un, const V3<T>& Up, T tol_h, T g)
+// The momentum flux u q + g h^2 / 2 of one side. PIN states which product is fused with the
+// sum: u q, or (gh) g h / 2 h; left to the compiler (PIN = false) it depends on the code around.
+template <typename T, bool PIN> MW_HD T momentum_flux(T u, T q, T h, T g, bool gh)
+{
+    if constexpr (PIN) return gh ? fma(T(0.5) * g * h, h, u * q) : fma(u, q, T(0.5) * g * h * h);
+    else return u * q + T(0.5) * g * h * h;
+}
+template <typename T, bool PIN = false>
+MW_HD V3<T> flux_hll_x(const V3<T>& Un, const V3<T>& Up, T tol_h, T g, bool gh_neg = false, bool gh_pos = false)
 {
     if (Un.h < tol_h && Up.h < tol_h) return {T(0), T(0), T(0)};
     const T h_neg = (Un.h < tol_h) ? T(0.0) : Un.h;
@@ -245,8 +248,8 @@ template <typename T> MW_HD V3<T> flux_hll_x(const V3<T>& Un, const V3<T>& Up, T
     const T a_star = sqrt(g * h_star);
     const T s_neg = (h_neg < tol_h) ? u_pos - T(2.0) * a_pos : fmin(u_neg - a_neg, u_star - a_star);
     const T s_pos = (h_pos < tol_h) ? u_neg + T(2.0) * a_neg : fmax(u_pos + a_pos, u_star + a_star);
-    const V3<T> F_neg = {Un.qx, u_neg * Un.qx + T(0.5) * g * h_neg * h_neg, Un.qy * u_neg};
-    const V3<T> F_pos = {Up.qx, u_pos * Up.qx + T(0.5) * g * h_pos * h_pos, Up.qy * u_pos};
+    const V3<T> F_neg = {Un.qx, momentum_flux<T, PIN>(u_neg, Un.qx, h_neg, g, gh_neg), Un.qy * u_neg};
+    const V3<T> F_pos = {Up.qx, momentum_flux<T, PIN>(u_pos, Up.qx, h_pos, g, gh_pos), Up.qy * u_pos};
     if (s_neg >= T(0.0)) return F_neg;
     if (s_neg < T(0.0) && s_pos >= T(0.0))
     {
@@ -298,33 +301,5 @@ template <typename T> MW_HD T minmod(T a, T b, T c)
 
 // zorder/get_x_coord.cuh, get_y_coord.cuh, get_spatial_coord.cuh (cell centre)
 template <typename T> MW_HD T cell_centre(int i, T d_loc) { return i * d_loc + d_loc / T(2.0); }
-
-// Direction codes of types/Directions.h
-enum Dir : int { NORTH = 1, EAST = 2, SOUTH = 4, WEST = 8 };
-
-// operators/get_leg_basis.cuh:12-40 with get_{x,y}_face_{coord,unit}.cuh.
-// (x, y): centre of the local cell; (xn, yn, dn): centre and size of the neighbour
-// (unused when nb_is_border).
-template <typename T, int DIR>
-MW_HD P3<T> leg_basis(bool nb_is_border, T x, T y, T dx_loc, T dy_loc, T xn, T yn, T dxn, T dyn)
-{
-    T x_face, y_face;
-    if (DIR == NORTH) { x_face = x - dx_loc / T(2.0) + T(0.5) * dx_loc; y_face = y - dy_loc / T(2.0) + T(1.0) * dy_loc; }
-    else if (DIR == SOUTH) { x_face = x - dx_loc / T(2.0) + T(0.5) * dx_loc; y_face = y - dy_loc / T(2.0) + T(0.0) * dy_loc; }
-    else if (DIR == EAST) { x_face = x - dx_loc / T(2.0) + T(1.0) * dx_loc; y_face = y - dy_loc / T(2.0) + T(0.5) * dy_loc; }
-    else { x_face = x - dx_loc / T(2.0) + T(0.0) * dx_loc; y_face = y - dy_loc / T(2.0) + T(0.5) * dy_loc; }
-    T xu, yu;
-    if (nb_is_border)
-    {
-        xu = (DIR == NORTH || DIR == SOUTH) ? T(0.5) : (DIR == EAST) ? T(0.0) : T(1.0);
-        yu = (DIR == EAST || DIR == WEST) ? T(0.5) : (DIR == NORTH) ? T(0.0) : T(1.0);
-    }
-    else
-    {
-        xu = (x_face - (xn - dxn / T(2.0))) / dxn;
-        yu = (y_face - (yn - dyn / T(2.0))) / dyn;
-    }
-    return {T(1.0), sqrt(T(3.0)) * (T(2.0) * xu - T(1.0)), sqrt(T(3.0)) * (T(2.0) * yu - T(1.0))};
-}
 
 } // namespace mw

@@ -136,9 +136,9 @@ __device__ __forceinline__ void ghost_pass(T& own_h0, T own_qx0, T own_qy0, T ow
 
 // operators/friction_implicit.cu:155-264 -- implicit friction on the mode-0 value and,
 // for MWDG2, on the four Gauss-point values, whose differences rebuild the slopes.
-// One out-of-line copy of the implicit Manning update of a point value (apply_friction);
-// a stage kernel applies it at 25 points per leaf (5 points of the leaf and of each of its
-// four neighbours) and would otherwise hold 25 inlined copies of its pow and divisions.
+// One out-of-line copy of the implicit Manning update of a point value (apply_friction):
+// the stage kernel applies it at up to 7 points per lane and would otherwise hold as many
+// inlined copies of its pow and divisions, which stall warps on instruction fetch.
 template <typename T> struct Q2 { T qx, qy; };
 template <typename T> __device__ __noinline__ Q2<T> friction_point(T h, T qx, T qy, T tol_h, T tol_s, T n, T g, T dt)
 {
@@ -146,193 +146,145 @@ template <typename T> __device__ __noinline__ Q2<T> friction_point(T h, T qx, T 
     return {qx, qy};
 }
 
-template <typename T, bool MW> __device__ __forceinline__ void friction_cell(Cell<T>& c, const Params<T>& P, T dt)
+// Friction of a first-order cell.
+template <typename T> __device__ __forceinline__ void friction_cell(Cell<T>& c, const Params<T>& P, T dt)
 {
-    if (!MW)
-    {
-        apply_friction(c.h[0], P.tol_h, P.tol_s, c.qx[0], c.qy[0], P.manning, P.g, dt);
-        return;
-    }
-    const T hlx = c.h[0] - c.h[1], hux = c.h[0] + c.h[1];
-    const T hly = c.h[0] - c.h[2], huy = c.h[0] + c.h[2];
-    T qxlx = c.qx[0] - c.qx[1], qxux = c.qx[0] + c.qx[1];
-    T qxly = c.qx[0] - c.qx[2], qxuy = c.qx[0] + c.qx[2];
-    T qylx = c.qy[0] - c.qy[1], qyux = c.qy[0] + c.qy[1];
-    T qyly = c.qy[0] - c.qy[2], qyuy = c.qy[0] + c.qy[2];
-    Q2<T> r = friction_point(c.h[0], c.qx[0], c.qy[0], P.tol_h, P.tol_s, P.manning, P.g, dt);
-    c.qx[0] = r.qx; c.qy[0] = r.qy;
-    r = friction_point(hlx, qxlx, qylx, P.tol_h, P.tol_s, P.manning, P.g, dt);
-    qxlx = r.qx; qylx = r.qy;
-    r = friction_point(hux, qxux, qyux, P.tol_h, P.tol_s, P.manning, P.g, dt);
-    qxux = r.qx; qyux = r.qy;
-    r = friction_point(hly, qxly, qyly, P.tol_h, P.tol_s, P.manning, P.g, dt);
-    qxly = r.qx; qyly = r.qy;
-    r = friction_point(huy, qxuy, qyuy, P.tol_h, P.tol_s, P.manning, P.g, dt);
-    qxuy = r.qx; qyuy = r.qy;
-    c.qx[1] = T(0.5) * (qxux - qxlx);
-    c.qx[2] = T(0.5) * (qxuy - qxly);
-    c.qy[1] = T(0.5) * (qyux - qylx);
-    c.qy[2] = T(0.5) * (qyuy - qyly);
+    apply_friction(c.h[0], P.tol_h, P.tol_s, c.qx[0], c.qy[0], P.manning, P.g, dt);
 }
 
-// What the limiter and the flux of a face need from one neighbour.
+// Friction of a DG2 cell's slopes along one axis: the point values at its two face centres
+// there (value -/+ slope), whose difference is the new slope.
+template <typename T>
+__device__ __forceinline__ void friction_slope(T h0, T qx0, T qy0, T hm, T& qxm, T& qym, const Params<T>& P, T dt)
+{
+    const Q2<T> lo = friction_point(h0 - hm, qx0 - qxm, qy0 - qym, P.tol_h, P.tol_s, P.manning, P.g, dt);
+    const Q2<T> hi = friction_point(h0 + hm, qx0 + qxm, qy0 + qym, P.tol_h, P.tol_s, P.manning, P.g, dt);
+    qxm = T(0.5) * (hi.qx - lo.qx);
+    qym = T(0.5) * (hi.qy - lo.qy);
+}
+
+// ---------------------------------------------------------------- DG2: two lanes per leaf
+//
+// Lane 0 of a pair takes the leaf's y axis (faces N and S), lane 1 its x axis (E and W). A lane
+// holds of the own cell mode 0 and the axis' slope mode (1y or 1x), which is all that the
+// axis' face values, limiter and friction points read, and writes fields as (h, n, t): the
+// depth, the discharge along the axis and the one across it, so both lanes run one code.
+
+// A lane's arrays, chosen without indexing the parameter block by a runtime value.
+template <typename T> struct Axis
+{
+    T *h0, *hm, *n0, *nm, *t0, *tm;   // modes 0 and m (the axis' slope) of h (or eta), n and t
+};
+template <typename T> __device__ __forceinline__ Axis<T> axis_of(const Hier<T>& h, bool x)
+{
+    return {h.s[0][0], x ? h.s[0][1] : h.s[0][2], x ? h.s[1][0] : h.s[2][0], x ? h.s[1][1] : h.s[2][2],
+            x ? h.s[2][0] : h.s[1][0], x ? h.s[2][1] : h.s[1][2]};
+}
+template <typename T> __device__ __forceinline__ Axis<T> axis_of(const Leaves<T>& l, bool x)
+{
+    return {l.un[0], x ? l.un[1] : l.un[2], x ? l.un[3] : l.un[6], x ? l.un[4] : l.un[8],
+            x ? l.un[6] : l.un[3], x ? l.un[7] : l.un[5]};
+}
+
+// Friction of a point value in a lane's (n, t) order.
+template <typename T>
+__device__ __forceinline__ void friction_axis(bool x, T h, T& n, T& t, const Params<T>& P, T dt)
+{
+    const Q2<T> r = friction_point(h, x ? n : t, x ? t : n, P.tol_h, P.tol_s, P.manning, P.g, dt);
+    n = x ? r.qx : r.qy;
+    t = x ? r.qy : r.qx;
+}
+
+// Friction of a cell's slope along one axis: the point values at its two face centres there
+// (value -/+ slope), whose half difference is the new slope.
+template <typename T>
+__device__ __forceinline__ void friction_slope(bool x, T h0, T n0, T t0, T hm, T& nm, T& tm, const Params<T>& P, T dt)
+{
+    T ln = n0 - nm, lt = t0 - tm, un = n0 + nm, ut = t0 + tm;
+    friction_axis(x, h0 - hm, ln, lt, P, dt);
+    friction_axis(x, h0 + hm, un, ut, P, dt);
+    nm = T(0.5) * (un - ln);
+    tm = T(0.5) * (ut - lt);
+}
+
+// What the limiter and the flux of a face need from its neighbour: the values at the face
+// (suffix f) and mode 0.
 template <typename T> struct NbFace
 {
-    T h0, eta0, qx0, qy0;   // mode-0 values
-    T hf, qxf, qyf, zf;     // values at the shared face (neighbour's Legendre basis)
-    T etaf;                 // face value of eta = z + h (limiter)
+    T h0, n0, t0, z0, hf, nf, tf, zf, etaf;
 };
 
-template <typename T> __device__ __forceinline__ NbFace<T> nb_face(const Cell<T>& c, const P3<T>& b)
+// The neighbour `nid` (level nlvl; -1: the ghost cell with depth gh and discharges gn, gt over
+// the own bed z0, slopes zero) across the high (N, E) or low (S, W) face of a leaf centred
+// at (xc, yc): its coefficients, rubbed when `fric`, at the shared face
+// (operators/get_leg_basis.cuh:12-40 with get_{x,y}_face_{coord,unit}.cuh).
+template <typename T>
+__device__ __forceinline__ NbFace<T> neighbour(const Hier<T>& hr, const Axis<T>& A, bool x, bool high, int nid, int nlvl, T gh,
+                                               T gn, T gt, T z0, T xc, T yc, T dxl, bool fric, const Params<T>& P, T dt)
 {
+    // c*[0]: mode 0, c*[1]: the slope along the axis, c*[2]: across it
+    T h[3], n[3], t[3], z[3], bm, bt;
+    if (nid != -1)
+    {
+        const T dn = P.dx * (1 << (P.L - nlvl));
+        const int code = nid - lvl_idx(nlvl);
+        // the face centre and the neighbour's centre along the axis (a) and across it (c)
+        const T a = x ? xc : yc, c = x ? yc : xc;
+        const T an = cell_centre(compact(x ? code : code >> 1), dn), cn = cell_centre(compact(x ? code >> 1 : code), dn);
+        const T a_face = a - dxl / T(2.0) + (high ? T(1.0) : T(0.0)) * dxl, c_face = c - dxl / T(2.0) + T(0.5) * dxl;
+        bm = sqrt(T(3.0)) * (T(2.0) * ((a_face - (an - dn / T(2.0))) / dn) - T(1.0));
+        bt = sqrt(T(3.0)) * (T(2.0) * ((c_face - (cn - dn / T(2.0))) / dn) - T(1.0));
+        const T* const zm = x ? hr.s[3][1] : hr.s[3][2];
+        const T* const zt = x ? hr.s[3][2] : hr.s[3][1];
+        const T* const ht = x ? hr.s[0][2] : hr.s[0][1];
+        const T* const nt = x ? hr.s[1][2] : hr.s[2][1];
+        const T* const tt = x ? hr.s[2][2] : hr.s[1][1];
+        z[0] = hr.s[3][0][nid]; z[1] = zm[nid]; z[2] = zt[nid];
+        h[0] = A.h0[nid] - z[0]; h[1] = A.hm[nid] - z[1]; h[2] = ht[nid] - z[2];
+        n[0] = A.n0[nid]; n[1] = A.nm[nid]; n[2] = nt[nid];
+        t[0] = A.t0[nid]; t[1] = A.tm[nid]; t[2] = tt[nid];
+    }
+    else
+    {
+        bm = bt = T(0.0);
+        z[0] = z0; h[0] = gh; n[0] = gn; t[0] = gt;
+        z[1] = z[2] = h[1] = h[2] = n[1] = n[2] = t[1] = t[2] = T(0.0);
+    }
+    if (fric)
+    {
+        T rn = n[0], rt = t[0];
+        friction_axis(x, h[0], rn, rt, P, dt);
+        // points along the face only where the basis there is not zero (a neighbour of
+        // another size): the slope they give is otherwise multiplied by zero
+        if (bm != T(0.0)) friction_slope(x, h[0], n[0], t[0], h[1], n[1], t[1], P, dt);
+        if (bt != T(0.0)) friction_slope(x, h[0], n[0], t[0], h[2], n[2], t[2], P, dt);
+        n[0] = rn; t[0] = rt;
+    }
     NbFace<T> r;
-    r.h0 = c.h[0];
-    r.qx0 = c.qx[0];
-    r.qy0 = c.qy[0];
-    r.eta0 = c.z[0] + c.h[0];
-    r.hf = face(P3<T>{c.h[0], c.h[1], c.h[2]}, b);
-    r.qxf = face(P3<T>{c.qx[0], c.qx[1], c.qx[2]}, b);
-    r.qyf = face(P3<T>{c.qy[0], c.qy[1], c.qy[2]}, b);
-    r.zf = face(P3<T>{c.z[0], c.z[1], c.z[2]}, b);
-    r.etaf = face(P3<T>{c.z[0] + c.h[0], c.z[1] + c.h[1], c.z[2] + c.h[2]}, b);
+    r.h0 = h[0]; r.n0 = n[0]; r.t0 = t[0]; r.z0 = z[0];
+    // modes in the order 0, 1x, 1y, as the reference sums them
+    const T bx = x ? bm : bt, by = x ? bt : bm;
+    auto at = [&](const T (&v)[3]) { return face(P3<T>{v[0], x ? v[1] : v[2], x ? v[2] : v[1]}, P3<T>{T(1.0), bx, by}); };
+    r.hf = at(h); r.nf = at(n); r.tf = at(t); r.zf = at(z);
+    const T e[3] = {z[0] + h[0], z[1] + h[1], z[2] + h[2]};
+    r.etaf = at(e);
     return r;
 }
 
-// operators/get_limited_slopes.cuh:10-78 for one field u (own planar coefficients),
-// given the neighbours' face values and mode-0 values of that field.
+// Limited slope of one field along the lane's axis (operators/get_limited_slopes.cuh:10-78):
+// u0, um the own coefficients; hf, lf and h0, l0 the high and low neighbours' face values and
+// mode 0. The x differences are divided by sqrt(3), as the reference does.
 template <typename T>
-__device__ __forceinline__ void limited_slopes(const P3<T>& u, T un_pos, T ue_pos, T us_neg, T uw_neg, T un0, T ue0, T us0,
-                                               T uw0, T dxf, T tolK, T& o1x, T& o1y)
+__device__ __forceinline__ T limited_slope(bool x, T u0, T um, T hf, T lf, T h0, T l0, T dxf, T tolK)
 {
     const T s3 = sqrt(T(3.0));
-    const T u_n_neg = face(u, P3<T>{T(1.0), T(0.0), s3});
-    const T u_e_neg = face(u, P3<T>{T(1.0), s3, T(0.0)});
-    const T u_s_pos = face(u, P3<T>{T(1.0), T(0.0), -s3});
-    const T u_w_pos = face(u, P3<T>{T(1.0), -s3, T(0.0)});
-    const T jn = fabs(un_pos - u_n_neg);
-    const T je = fabs(ue_pos - u_e_neg);
-    const T js = fabs(u_s_pos - us_neg);
-    const T jw = fabs(u_w_pos - uw_neg);
-    const T norm_x = fmax(fabs(u._0 - u._1x), fabs(u._0 + u._1x));
-    const T norm_y = fmax(fabs(u._0 - u._1y), fabs(u._0 + u._1y));
-    const T DS_e = (norm_x > T(1e-12)) ? je / (T(0.5) * dxf * norm_x) : T(0.0);
-    const T DS_w = (norm_x > T(1e-12)) ? jw / (T(0.5) * dxf * norm_x) : T(0.0);
-    const T DS_n = (norm_y > T(1e-12)) ? jn / (T(0.5) * dxf * norm_y) : T(0.0);
-    const T DS_s = (norm_y > T(1e-12)) ? js / (T(0.5) * dxf * norm_y) : T(0.0);
-    o1x = (fmax(DS_e, DS_w) < tolK) ? u._1x : minmod(u._1x, (u._0 - uw0) / s3, (ue0 - u._0) / s3);
-    o1y = (fmax(DS_n, DS_s) < tolK) ? u._1y : minmod(u._1y, (u._0 - us0), (un0 - u._0));
-}
-
-template <typename T> struct Geo { T x, y, dxl; bool in_extent; };
-
-template <typename T> __device__ __forceinline__ Geo<T> leaf_geo(int act, int level, const Params<T>& P)
-{
-    Geo<T> g;
-    g.dxl = P.dx * (1 << (P.L - level));
-    const int code = act - lvl_idx(level);
-    g.x = cell_centre(compact(code), g.dxl);
-    g.y = cell_centre(compact(code >> 1), g.dxl);
-    g.in_extent = !((g.x >= P.xsz * P.dx) || (g.y >= P.ysz * P.dx));
-    return g;
-}
-
-// Legendre basis of the neighbour in direction D evaluated at the shared face.
-template <typename T, int DIR>
-__device__ __forceinline__ P3<T> nb_basis(const Geo<T>& g, int nid, int nlvl, const Params<T>& P)
-{
-    if (nid == -1) return leg_basis<T, DIR>(true, g.x, g.y, g.dxl, g.dxl, T(0), T(0), T(1), T(1));
-    const T dn = P.dx * (1 << (P.L - nlvl));
-    const int code = nid - lvl_idx(nlvl);
-    const T xn = cell_centre(compact(code), dn);
-    const T yn = cell_centre(compact(code >> 1), dn);
-    return leg_basis<T, DIR>(false, g.x, g.y, g.dxl, g.dxl, xn, yn, dn, dn);
-}
-
-// operators/dg2_update.cu:160-334 -- the DG2 right-hand side applied to the own
-// coefficients c (h, qx, qy planar; z planar) with the neighbours' face values.
-template <typename T>
-__device__ __forceinline__ void dg2_rhs_update(const P3<T>& ch, const P3<T>& cqx, const P3<T>& cqy, const P3<T>& zp,
-                                               const NbFace<T> (&nf)[4], T dxl, const Params<T>& P, T dt, T (&out)[9])
-{
-    const T s3 = sqrt(T(3.0));
-    const T g = P.g, tol_h = P.tol_h;
-    const P3<T> bn = {T(1.0), T(0.0), s3}, be = {T(1.0), s3, T(0.0)};
-    const P3<T> bs = {T(1.0), T(0.0), -s3}, bw = {T(1.0), -s3, T(0.0)};
-    const T z_n_pos = nf[0].zf, z_e_pos = nf[1].zf, z_s_neg = nf[2].zf, z_w_neg = nf[3].zf;
-    const T z_n_neg = face(zp, bn), z_e_neg = face(zp, be), z_s_pos = face(zp, bs), z_w_pos = face(zp, bw);
-    const T zi_n = fmax(z_n_neg, z_n_pos), zi_e = fmax(z_e_neg, z_e_pos);
-    const T zi_s = fmax(z_s_neg, z_s_pos), zi_w = fmax(z_w_neg, z_w_pos);
-    const V3<T> Us_n_pos = star(V3<T>{nf[0].hf, nf[0].qxf, nf[0].qyf}, z_n_pos, zi_n, tol_h);
-    const V3<T> Us_e_pos = star(V3<T>{nf[1].hf, nf[1].qxf, nf[1].qyf}, z_e_pos, zi_e, tol_h);
-    const V3<T> Us_s_neg = star(V3<T>{nf[2].hf, nf[2].qxf, nf[2].qyf}, z_s_neg, zi_s, tol_h);
-    const V3<T> Us_w_neg = star(V3<T>{nf[3].hf, nf[3].qxf, nf[3].qyf}, z_w_neg, zi_w, tol_h);
-    const T hfn = face(ch, bn), hfe = face(ch, be), hfs = face(ch, bs), hfw = face(ch, bw);
-    const V3<T> Us_n_neg = star(V3<T>{hfn, face(cqx, bn), face(cqy, bn)}, z_n_neg, zi_n, tol_h);
-    const V3<T> Us_e_neg = star(V3<T>{hfe, face(cqx, be), face(cqy, be)}, z_e_neg, zi_e, tol_h);
-    const V3<T> Us_s_pos = star(V3<T>{hfs, face(cqx, bs), face(cqy, bs)}, z_s_pos, zi_s, tol_h);
-    const V3<T> Us_w_pos = star(V3<T>{hfw, face(cqx, bw), face(cqy, bw)}, z_w_pos, zi_w, tol_h);
-    const V3<T> F_n = flux_hll_y(Us_n_neg, Us_n_pos, tol_h, g);
-    const V3<T> F_e = flux_hll_x(Us_e_neg, Us_e_pos, tol_h, g);
-    const V3<T> F_s = flux_hll_y(Us_s_neg, Us_s_pos, tol_h, g);
-    const V3<T> F_w = flux_hll_x(Us_w_neg, Us_w_pos, tol_h, g);
-    // x direction: modes 0 and 1x (operators/get_bed_src.cuh:46-72 for the bed slope)
-    const V3<T> U0x = (Us_e_neg + Us_w_pos) / T(2.0);
-    const V3<T> U1x = (Us_e_neg - Us_w_pos) / (T(2.0) * s3);
-    V3<T> Lx0 = (-T(1.0) * (F_e - F_w)) / dxl;
-    V3<T> Lx1 = (-s3 / dxl) * (F_e + F_w - phys_flux_x(U0x - U1x, tol_h, g) - phys_flux_x(U0x + U1x, tol_h, g));
-    {
-        const T eta_e_neg = hfe + z_e_neg, eta_w_pos = hfw + z_w_pos;
-        const T zse = zi_e - fmax(T(0.0), -(eta_e_neg - zi_e));
-        const T zsw = zi_w - fmax(T(0.0), -(eta_w_pos - zi_w));
-        const T z1 = (zse - zsw) / (T(2.0) * s3);
-        Lx0.qx = Lx0.qx + -T(2.0) * s3 * g * U0x.h * z1 / dxl;
-        Lx1.qx = Lx1.qx + -T(2.0) * s3 * g * U1x.h * z1 / dxl;
-        Lx0.h = Lx0.h + T(0.0); Lx0.qy = Lx0.qy + T(0.0);
-        Lx1.h = Lx1.h + T(0.0); Lx1.qy = Lx1.qy + T(0.0);
-    }
-    // y direction: modes 0 and 1y
-    const V3<T> U0y = (Us_n_neg + Us_s_pos) / T(2.0);
-    const V3<T> U1y = (Us_n_neg - Us_s_pos) / (T(2.0) * s3);
-    V3<T> Ly0 = (-T(1.0) * (F_n - F_s)) / dxl;
-    V3<T> Ly1 = (-s3 / dxl) * (F_s + F_n - phys_flux_y(U0y - U1y, tol_h, g) - phys_flux_y(U0y + U1y, tol_h, g));
-    {
-        const T eta_n_neg = hfn + z_n_neg, eta_s_pos = hfs + z_s_pos;
-        const T zsn = zi_n - fmax(T(0.0), -(eta_n_neg - zi_n));
-        const T zss = zi_s - fmax(T(0.0), -(eta_s_pos - zi_s));
-        const T z1 = (zsn - zss) / (T(2.0) * s3);
-        Ly0.qy = Ly0.qy + -T(2.0) * s3 * g * U0y.h * z1 / dxl;
-        Ly1.qy = Ly1.qy + -T(2.0) * s3 * g * U1y.h * z1 / dxl;
-        Ly0.h = Ly0.h + T(0.0); Ly0.qx = Ly0.qx + T(0.0);
-        Ly1.h = Ly1.h + T(0.0); Ly1.qx = Ly1.qx + T(0.0);
-    }
-    // coeffs += dt * (Lx + Ly): Lx has modes (0, 1x, 0), Ly has (0, 0, 1y)
-    const T zero = T(0.0);
-    out[0] = ch._0 + dt * (Lx0.h + Ly0.h);
-    out[1] = ch._1x + dt * (Lx1.h + zero);
-    out[2] = ch._1y + dt * (zero + Ly1.h);
-    out[3] = cqx._0 + dt * (Lx0.qx + Ly0.qx);
-    out[4] = cqx._1x + dt * (Lx1.qx + zero);
-    out[5] = cqx._1y + dt * (zero + Ly1.qx);
-    out[6] = cqy._0 + dt * (Lx0.qy + Ly0.qy);
-    out[7] = cqy._1x + dt * (Lx1.qy + zero);
-    out[8] = cqy._1y + dt * (zero + Ly1.qy);
-}
-
-// Depth after ghost cells of the own leaf and its four neighbours; a leaf is dry when all
-// five are below tol_h: it is not updated (dg2_update.cu:36-50), not limited (the limiter
-// needs a depth above 0.05 max_h) and, being below tol_h, gets no friction, so it needs
-// none of its neighbours' other coefficients.
-template <typename T>
-__device__ __forceinline__ bool leaf_is_dry(const Hier<T>& hr, T own_h0, const int32_t (&nid)[4], const T (&gh)[4], T tol_h)
-{
-    if (!(own_h0 < tol_h)) return false;
-#pragma unroll
-    for (int d = 0; d < 4; ++d)
-    {
-        const T h = (nid[d] != -1) ? hr.s[0][0][nid[d]] - hr.s[3][0][nid[d]] : gh[d];
-        if (!(h < tol_h)) return false;
-    }
-    return true;
+    const T jh = fabs(hf - (u0 + um * s3)), jl = fabs((u0 - um * s3) - lf);
+    const T norm = fmax(fabs(u0 - um), fabs(u0 + um));
+    const T dh = (norm > T(1e-12)) ? jh / (T(0.5) * dxf * norm) : T(0.0);
+    const T dl = (norm > T(1e-12)) ? jl / (T(0.5) * dxf * norm) : T(0.0);
+    T a = u0 - l0, b = h0 - u0;
+    if (x) { a = a / s3; b = b / s3; }
+    return fmax(dh, dl) < tolK ? um : minmod(um, a, b);
 }
 
 // Leaf state u (h, qx, qy by mode, the layout of Leaves::un) into the hierarchy at `a`,
@@ -356,12 +308,12 @@ __device__ __forceinline__ void put_leaf(const Hier<T>& hr, int a, const T (&u)[
 template <typename T> struct StateMax
 {
     T eta = T(0), h = T(0), qx = T(0), z = T(0);
-    __device__ __forceinline__ void add(const T (&u)[9], T z0)
+    __device__ __forceinline__ void add(T h0, T qx0, T z0)
     {
-        const T e = u[0] + z0;
+        const T e = h0 + z0;
         eta = fmax(eta, fabs(e));
-        h = fmax(h, fabs(u[0]));
-        qx = fmax(qx, fabs(u[3]));
+        h = fmax(h, fabs(h0));
+        qx = fmax(qx, fabs(qx0));
         z = fmax(z, fabs(z0));
     }
     __device__ __forceinline__ void flush(Scalars<T>* sc)
@@ -381,8 +333,7 @@ __device__ __forceinline__ void put_leaf_fv1(const Hier<T>& hout, int a, T h, T 
     hout.s[0][0][a] = h + z;
     hout.s[1][0][a] = qx;
     hout.s[2][0][a] = qy;
-    const T u[9] = {h, T(0), T(0), qx, T(0), T(0), qy, T(0), T(0)};
-    mx.add(u, z);
+    mx.add(h, qx, z);
 }
 
 // Wet test of one RK stage (the rule of leaf_is_dry, after ghost cells): wet leaves are
@@ -511,10 +462,7 @@ __device__ __forceinline__ void k_stage_dry_body(int bid, int nb, Leaves<T> lf, 
             }
             if (STAGE == 2 && left_out && dry1[i] == 2)
             {
-                T u[9];
-                u[0] = lf.un[0][i];
-                u[3] = lf.un[3][i];
-                mx.add(u, hin.s[3][0][a]);
+                mx.add(lf.un[0][i], lf.un[3][i], hin.s[3][0][a]);
                 if (P.dt_leaf) P.dt_leaf[i] = P.initial_tstep;
                 continue;
             }
@@ -541,7 +489,7 @@ __device__ __forceinline__ void k_stage_dry_body(int bid, int nb, Leaves<T> lf, 
         {
 #pragma unroll
             for (int k = 0; k < 9; ++k) u[k] = lf.un[k][i];
-            mx.add(u, z[0]);
+            mx.add(u[0], u[3], z[0]);
             if (P.dt_leaf) P.dt_leaf[i] = P.initial_tstep;
         }
         put_leaf(hout, a, u, z, wmark);
@@ -561,6 +509,11 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 5) k_stage_dry(Leave
     k_stage_dry_body<T, STAGE>(blockIdx.x, gridDim.x, lf, hin, hout, sc, P, friction, dry, dry1, pm, clean_tag);
 }
 
+// Resident blocks of k_mwdg2_stage per SM that its registers are held to (64 in FP32, 128 in
+// FP64, with a few spills): 8 / 4 took 135.8 us for the dam-break step and 3.74 ms for the
+// ensemble's where 6 / 3 took 148.6 us and 3.94 ms; 9 / 5 and 10 / 6 are within noise of it.
+template <typename T> constexpr int kStageBlocks = sizeof(T) == 4 ? 8 : 4;
+
 // One RK2 stage of MWDG2, reading the hierarchy `hin` and writing each leaf's result into
 // the hierarchy `hout` at the leaf's own index (which no leaf reads in this stage).
 // STAGE 1 (hin: hierarchy, hout: stage hierarchy): friction (once per step), limiter with
@@ -569,174 +522,210 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 5) k_stage_dry(Leave
 // U^{n+1} = (U** + U^n)/2 -> un and hout (the next step's re-insertion,
 // mra/reinsert_assem_sol.cu), the next step's maxima, CFL dt. LIST: only the leaves in
 // the wet list built by k_stage_wet; otherwise every leaf.
+//
+// What bounds it: few wet leaves, one leaf's serial latency; many, instruction issue (IEEE
+// divisions, square roots and pow of the friction and the fluxes). Two lanes per leaf halve the
+// chain of a leaf without evaluating anything twice but its mean friction point and its own
+// mode-0 loads, and need about half the registers of a thread that holds all four faces.
+// Against one thread per leaf (ncu, per launch, stage 1 / 2): 256^2 dam break FP64, every leaf
+// wet, 33.3 / 33.7 -> 15.3 / 17.6 us; 1000 x 700 flood FP64 54.8 / 28.8 -> 34.5 / 23.1 us; wet
+// list of the 2048^2 urban case FP32 86.2 / 58.5 -> 74.9 / 56.3 us; step of eight ensemble
+// members FP32 3.90 -> 3.52 ms. Four lanes per leaf (a face each) evaluated too much twice
+// (dam break step 142 -> 158 us, ensemble 4.37 -> 4.96 ms where this form takes 3.74).
 template <typename T, int STAGE, bool LIST>
 __device__ __forceinline__ void k_mwdg2_stage_body(int bid, int nb, Leaves<T> lf, Hier<T> hin, Hier<T> hout, Scalars<T>* sc,
                                                                 Params<T> P, const StepArgs<T>* args, bool friction,
                                                                 const int32_t* wet)
 {
     const T dt = args->dt;
-    const Bnd<T>& B = args->B;
     const Hier<T>& hr = hin;
     StateMax<T> mx;
-    const int n = LIST ? sc->wet[STAGE - 1] : sc->n_leaves;
+    const int nl = LIST ? sc->wet[STAGE - 1] : sc->n_leaves;
     T dt_loc = (sizeof(T) == 8) ? T(1.0e308) : T(3.0e38);
     bool nan_seen = false;
     unsigned n_wet = 0;
     const T max_h = (STAGE == 1) ? fmax(T(1.0), sc->max_h) : sc->max_h2;
     const uint32_t wmark = (sc->step_tag << 1) | 1u;   // a written stage-hierarchy slot (Hier::tag)
-    for (int k = bid * blockDim.x + threadIdx.x; k < n; k += nb * blockDim.x)
+    const bool x = (threadIdx.x & 1) != 0;
+    const unsigned pair = 3u << (threadIdx.x & 30);
+    const T s3 = sqrt(T(3.0));
+    const Axis<T> A = axis_of(hr, x);
+    const int32_t* const nb_hi = x ? lf.nb[1] : lf.nb[0];
+    const int32_t* const nb_lo = x ? lf.nb[3] : lf.nb[2];
+    const int per = blockDim.x >> 1;
+    for (int k = bid * per + (threadIdx.x >> 1); k < nl; k += nb * per)
     {
         const int i = LIST ? wet[k] : k;
         const int a = lf.act[i];
         const int level = lf.lvl[i];
-        int32_t nid[4];
-        int nl[4];
-#pragma unroll
-        for (int d = 0; d < 4; ++d) { nid[d] = lf.nb[d][i]; nl[d] = nid[d] == -1 ? level : level_of(nid[d]); }
-        Cell<T> own;
-        load_cell<T, true>(hr, a, own);
+        const int id_hi = nb_hi[i], id_lo = nb_lo[i];
+        const T z0 = hr.s[3][0][a], zm = (x ? hr.s[3][1] : hr.s[3][2])[a];
+        T h0 = A.h0[a] - z0, hm = A.hm[a] - zm;
+        T n0 = A.n0[a], nm = A.nm[a], t0 = A.t0[a], tm = A.tm[a];
         // a NaN depth anywhere in the state (a dry-looking NaN leaf is never updated below)
-        nan_seen |= (own.h[0] != own.h[0]);
-        T gh[4], gqx[4], gqy[4];
-        ghost_pass(own.h[0], own.qx[0], own.qy[0], own.z[0], nid, level, a, P, B, dt, gh, gqx, gqy);
-        // Depths of the four neighbours (after ghost cells). A leaf whose own depth and
-        // neighbour depths are all below tol_h is not updated (dg2_update.cu:36-50), is not
-        // limited (the limiter needs a depth above 0.05 max_h) and, being below tol_h, gets
-        // no friction: it needs none of the neighbours' other coefficients.
-        const bool dry = !LIST && leaf_is_dry(hr, own.h[0], nid, gh, P.tol_h);
-        n_wet += dry ? 0 : 1;
+        nan_seen |= (h0 != h0);
+        // ghost cells of border faces; a border segment may also reset the own depth, in the
+        // order N, E, S, W, so both lanes of a border leaf walk all four faces
+        T gh_hi = T(0.0), gn_hi = T(0.0), gt_hi = T(0.0), gh_lo = T(0.0), gn_lo = T(0.0), gt_lo = T(0.0);
+        if (__ballot_sync(pair, id_hi == -1 || id_lo == -1))
+        {
+            const int o_hi = __shfl_xor_sync(pair, id_hi, 1), o_lo = __shfl_xor_sync(pair, id_lo, 1);
+            const int32_t n4[4] = {x ? o_hi : id_hi, x ? id_hi : o_hi, x ? o_lo : id_lo, x ? id_lo : o_lo};
+            T gh[4], gqx[4], gqy[4];
+            ghost_pass(h0, x ? n0 : t0, x ? t0 : n0, z0, n4, level, a, P, args->B, dt, gh, gqx, gqy);
+            gh_hi = x ? gh[1] : gh[0]; gn_hi = x ? gqx[1] : gqy[0]; gt_hi = x ? gqy[1] : gqx[0];
+            gh_lo = x ? gh[3] : gh[2]; gn_lo = x ? gqx[3] : gqy[2]; gt_lo = x ? gqy[3] : gqx[2];
+        }
+        // A leaf whose own depth and neighbour depths (after ghost cells) are all below tol_h
+        // is not updated (dg2_update.cu:36-50), is not limited (the limiter needs a depth
+        // above 0.05 max_h) and, being below tol_h, gets no friction: it needs none of the
+        // neighbours' other coefficients.
+        bool dry = false;
+        if (!LIST)
+        {
+            const T hh = id_hi != -1 ? hr.s[0][0][id_hi] - hr.s[3][0][id_hi] : gh_hi;
+            const T hl = id_lo != -1 ? hr.s[0][0][id_lo] - hr.s[3][0][id_lo] : gh_lo;
+            dry = __ballot_sync(pair, !(hh < P.tol_h) || !(hl < P.tol_h)) == 0 && h0 < P.tol_h;
+            n_wet += (dry || x) ? 0 : 1;
+        }
         // friction_implicit.cu:24-48: shallow or slow leaves lose their discharge and
         // skip friction (their neighbours' copies are then left untouched too)
         bool fric = false;
         if (STAGE == 1 && friction)
         {
-            const T h = own.h[0];
-            const bool below_depth = (h < P.tol_h);
-            const T ux = below_depth ? T(0.0) : own.qx[0] / h;
-            const T uy = below_depth ? T(0.0) : own.qy[0] / h;
-            const bool below_speed = (fabs(ux) < P.tol_s && fabs(uy) < P.tol_s);
-            if (below_depth || below_speed) { own.qx[0] = T(0.0); own.qy[0] = T(0.0); }
+            const bool below_depth = (h0 < P.tol_h);
+            const T un = below_depth ? T(0.0) : n0 / h0;
+            const T ut = below_depth ? T(0.0) : t0 / h0;
+            const bool below_speed = (fabs(un) < P.tol_s && fabs(ut) < P.tol_s);
+            if (below_depth || below_speed) { n0 = T(0.0); t0 = T(0.0); }
             fric = !(below_depth || below_speed);
-            if (fric) friction_cell<T, true>(own, P, dt);
+            if (fric)
+            {
+                T rn = n0, rt = t0;
+                friction_axis(x, h0, rn, rt, P, dt);
+                friction_slope(x, h0, n0, t0, hm, nm, tm, P, dt);
+                n0 = rn; t0 = rt;
+            }
         }
+        // leaf state in the lane's coefficients: the slopes by both lanes, mode 0 by lane 0
+        auto put = [&](T uh0, T un0, T ut0, T uhm, T unm, T utm) {
+            const Axis<T> O = axis_of(hout, x);
+            O.hm[a] = uhm + zm; O.nm[a] = unm; O.tm[a] = utm;
+            if (!x)
+            {
+                O.h0[a] = uh0 + z0; O.n0[a] = un0; O.t0[a] = ut0;
+                if (hout.tag) hout.tag[a] = wmark;   // the stage hierarchy of the keep-values decode
+            }
+        };
+        auto put_un = [&](T uh0, T un0, T ut0, T uhm, T unm, T utm) {
+            const Axis<T> U = axis_of(lf, x);
+            U.hm[i] = uhm; U.nm[i] = unm; U.tm[i] = utm;
+            if (!x) { U.h0[i] = uh0; U.n0[i] = un0; U.t0[i] = ut0; }
+        };
         if (dry)
         {
-            T u[9];
-            if (STAGE == 1)
-            {
-#pragma unroll
-                for (int m = 0; m < 3; ++m) { u[m] = own.h[m]; u[3 + m] = own.qx[m]; u[6 + m] = own.qy[m]; }
-#pragma unroll
-                for (int k = 0; k < 9; ++k) lf.un[k][i] = u[k];
-            }
+            if (STAGE == 1) { put_un(h0, n0, t0, hm, nm, tm); put(h0, n0, t0, hm, nm, tm); }
             else
             {
-#pragma unroll
-                for (int k = 0; k < 9; ++k) u[k] = lf.un[k][i];
-                mx.add(u, own.z[0]);
+                const Axis<T> U = axis_of(lf, x);
+                const T uh = U.h0[i], un = U.n0[i], ut = U.t0[i];
+                if (!x)
+                {
+                    mx.add(uh, ut, z0);   // (t is qx in the y lane)
+                    if (P.dt_leaf) P.dt_leaf[i] = P.initial_tstep;
+                }
+                put(uh, un, ut, U.hm[i], U.nm[i], U.tm[i]);
             }
-            put_leaf(hout, a, u, own.z, wmark);
-            if (STAGE == 2 && P.dt_leaf) P.dt_leaf[i] = P.initial_tstep;
             dt_loc = fmin(dt_loc, P.initial_tstep);
             continue;
         }
-        const Geo<T> geo = leaf_geo<T>(a, level, P);
-        NbFace<T> nf[4];
-#pragma unroll
-        for (int d = 0; d < 4; ++d)
-        {
-            Cell<T> c;
-            if (nid[d] != -1) load_cell<T, true>(hr, nid[d], c);
-            else
-            {
-                c.h[0] = gh[d]; c.qx[0] = gqx[d]; c.qy[0] = gqy[d]; c.z[0] = own.z[0];
-                c.h[1] = c.h[2] = c.qx[1] = c.qx[2] = c.qy[1] = c.qy[2] = c.z[1] = c.z[2] = T(0.0);
-            }
-            if (fric) friction_cell<T, true>(c, P, dt);
-            P3<T> b;
-            if (d == 0) b = nb_basis<T, NORTH>(geo, nid[d], nl[d], P);
-            else if (d == 1) b = nb_basis<T, EAST>(geo, nid[d], nl[d], P);
-            else if (d == 2) b = nb_basis<T, SOUTH>(geo, nid[d], nl[d], P);
-            else b = nb_basis<T, WEST>(geo, nid[d], nl[d], P);
-            nf[d] = nb_face(c, b);
-        }
+        const T dxl = P.dx * (1 << (P.L - level));
+        const int code = a - lvl_idx(level);
+        const T xc = cell_centre(compact(code), dxl), yc = cell_centre(compact(code >> 1), dxl);
+        const bool in_extent = !((xc >= P.xsz * P.dx) || (yc >= P.ysz * P.dx));
+        const NbFace<T> H = neighbour(hr, A, x, true, id_hi, id_hi == -1 ? level : level_of(id_hi), gh_hi, gn_hi, gt_hi, z0, xc, yc,
+                                      dxl, STAGE == 1 && fric, P, dt);
+        const NbFace<T> W = neighbour(hr, A, x, false, id_lo, id_lo == -1 ? level : level_of(id_lo), gh_lo, gn_lo, gt_lo, z0, xc, yc,
+                                      dxl, STAGE == 1 && fric, P, dt);
         // operators/copy_to_buf_assem_sol.cu: the stage-1 result of a leaf that is not
         // updated is its state before limiting
-        T pre[9];
-        if (STAGE == 1)
-        {
-#pragma unroll
-            for (int m = 0; m < 3; ++m) { pre[m] = own.h[m]; pre[3 + m] = own.qx[m]; pre[6 + m] = own.qy[m]; }
-        }
+        const T pre_h = hm, pre_n = nm, pre_t = tm;
         // operators/limit_slopes.cu:3-238 (finest-level leaves inside the DEM only)
-        if (P.limit && level == P.L && geo.in_extent)
+        if (P.limit && level == P.L && in_extent)
         {
-            const P3<T> eta = {own.z[0] + own.h[0], own.z[1] + own.h[1], own.z[2] + own.h[2]};
-            const P3<T> qx = {own.qx[0], own.qx[1], own.qx[2]}, qy = {own.qy[0], own.qy[1], own.qy[2]};
-            T e1x, e1y, q1x, q1y, r1x, r1y;
-            limited_slopes(eta, nf[0].etaf, nf[1].etaf, nf[2].etaf, nf[3].etaf, nf[0].eta0, nf[1].eta0, nf[2].eta0,
-                           nf[3].eta0, P.dx, P.tol_Krivo, e1x, e1y);
-            limited_slopes(qx, nf[0].qxf, nf[1].qxf, nf[2].qxf, nf[3].qxf, nf[0].qx0, nf[1].qx0, nf[2].qx0, nf[3].qx0,
-                           P.dx, P.tol_Krivo, q1x, q1y);
-            limited_slopes(qy, nf[0].qyf, nf[1].qyf, nf[2].qyf, nf[3].qyf, nf[0].qy0, nf[1].qy0, nf[2].qy0, nf[3].qy0,
-                           P.dx, P.tol_Krivo, r1x, r1y);
-            const bool ax = (T(0.05) * max_h < fmin(own.h[0], fmin(nf[1].h0, nf[3].h0)));
-            const bool ay = (T(0.05) * max_h < fmin(own.h[0], fmin(nf[0].h0, nf[2].h0)));
-            if (ax) { own.h[1] = e1x - own.z[1]; own.qx[1] = q1x; own.qy[1] = r1x; }
-            if (ay) { own.h[2] = e1y - own.z[2]; own.qx[2] = q1y; own.qy[2] = r1y; }
+            const T e = limited_slope(x, z0 + h0, zm + hm, H.etaf, W.etaf, H.z0 + H.h0, W.z0 + W.h0, P.dx, P.tol_Krivo);
+            const T p = limited_slope(x, n0, nm, H.nf, W.nf, H.n0, W.n0, P.dx, P.tol_Krivo);
+            const T q = limited_slope(x, t0, tm, H.tf, W.tf, H.t0, W.t0, P.dx, P.tol_Krivo);
+            if (T(0.05) * max_h < fmin(h0, fmin(H.h0, W.h0))) { hm = e - zm; nm = p; tm = q; }
         }
-        if (STAGE == 1)
-        {
-#pragma unroll
-            for (int m = 0; m < 3; ++m) { lf.un[m][i] = own.h[m]; lf.un[3 + m][i] = own.qx[m]; lf.un[6 + m][i] = own.qy[m]; }
-        }
+        if (STAGE == 1) put_un(h0, n0, t0, hm, nm, tm);
         // operators/dg2_update.cu:31-79 (wet leaves, not high wall, inside the DEM)
-        const bool highwall = (fabs(own.z[0] - P.wall_height) < T(1e-10));
-        const bool wet = (own.h[0] >= P.tol_h || nf[0].h0 >= P.tol_h || nf[1].h0 >= P.tol_h || nf[2].h0 >= P.tol_h ||
-                          nf[3].h0 >= P.tol_h) && !highwall;
+        const bool highwall = (fabs(z0 - P.wall_height) < T(1e-10));
+        const bool any = h0 >= P.tol_h || __ballot_sync(pair, H.h0 >= P.tol_h || W.h0 >= P.tol_h) != 0;
         T leaf_dt = P.initial_tstep;
-        if (wet && geo.in_extent)
+        if (any && !highwall && in_extent)
         {
             // the leaf changes: the encode of the next step revisits its subtree
-            if (P.act && level >= P.act_level) P.act[(a - lvl_idx(level)) >> (2 * (level - P.act_level))] = 1;
-            T u[9];
-            dg2_rhs_update(P3<T>{own.h[0], own.h[1], own.h[2]}, P3<T>{own.qx[0], own.qx[1], own.qx[2]},
-                           P3<T>{own.qy[0], own.qy[1], own.qy[2]}, P3<T>{own.z[0], own.z[1], own.z[2]}, nf, geo.dxl, P, dt, u);
+            if (!x && P.act && level >= P.act_level) P.act[(a - lvl_idx(level)) >> (2 * (level - P.act_level))] = 1;
+            // operators/dg2_update.cu:160-334 along the axis
+            const T g = P.g, tol_h = P.tol_h;
+            const T hf_h = h0 + hm * s3, hf_l = h0 - hm * s3, zf_h = z0 + zm * s3, zf_l = z0 - zm * s3;
+            const T zi_h = fmax(zf_h, H.zf), zi_l = fmax(zf_l, W.zf);
+            const V3<T> s_h = star(V3<T>{hf_h, n0 + nm * s3, t0 + tm * s3}, zf_h, zi_h, tol_h);
+            const V3<T> s_l = star(V3<T>{hf_l, n0 - nm * s3, t0 - tm * s3}, zf_l, zi_l, tol_h);
+            // (the flux's tangential component changes sign with the tangential discharge, so
+            // the y lane needs no rotation of its frame)
+            // The fused products are stated: the one-thread form of this kernel, whose bits agree
+            // with the reference's build, fused u q everywhere but for the neighbours' side of
+            // the x faces (found by comparing all choices over dam breaks, catchments and floods
+            // in both precisions; this one gives the same bits everywhere).
+            const V3<T> F_h = flux_hll_x<T, true>(s_h, star(V3<T>{H.hf, H.nf, H.tf}, H.zf, zi_h, tol_h), tol_h, g, false, x);
+            const V3<T> F_l = flux_hll_x<T, true>(star(V3<T>{W.hf, W.nf, W.tf}, W.zf, zi_l, tol_h), s_l, tol_h, g, x, false);
+            const V3<T> U0 = (s_h + s_l) / T(2.0);
+            const V3<T> U1 = (s_h - s_l) / (T(2.0) * s3);
+            V3<T> L0 = (-T(1.0) * (F_h - F_l)) / dxl;
+            V3<T> L1 = (-s3 / dxl) * (F_h + F_l - phys_flux_x(U0 - U1, tol_h, g) - phys_flux_x(U0 + U1, tol_h, g));
+            // operators/get_bed_src.cuh:46-72
+            const T zs_h = zi_h - fmax(T(0.0), -((hf_h + zf_h) - zi_h));
+            const T zs_l = zi_l - fmax(T(0.0), -((hf_l + zf_l) - zi_l));
+            const T z1 = (zs_h - zs_l) / (T(2.0) * s3);
+            L0.qx = L0.qx + -T(2.0) * s3 * g * U0.h * z1 / dxl;
+            L1.qx = L1.qx + -T(2.0) * s3 * g * U1.h * z1 / dxl;
+            // coeffs += dt * (Lx + Ly): mode 0 takes both axes, a slope its own
+            const T oh = __shfl_xor_sync(pair, L0.h, 1);
+            const T on = __shfl_xor_sync(pair, L0.qy, 1), ot = __shfl_xor_sync(pair, L0.qx, 1);
+            T uh0 = h0 + dt * (L0.h + oh), un0 = n0 + dt * (L0.qx + on), ut0 = t0 + dt * (L0.qy + ot);
+            T uhm = hm + dt * L1.h, unm = nm + dt * L1.qx, utm = tm + dt * L1.qy;
             if (STAGE == 2)
             {
-#pragma unroll
-                for (int k = 0; k < 9; ++k) u[k] = T(0.5) * (u[k] + lf.un[k][i]);
+                const Axis<T> U = axis_of(lf, x);
+                uh0 = T(0.5) * (uh0 + U.h0[i]); un0 = T(0.5) * (un0 + U.n0[i]); ut0 = T(0.5) * (ut0 + U.t0[i]);
+                uhm = T(0.5) * (uhm + U.hm[i]); unm = T(0.5) * (unm + U.nm[i]); utm = T(0.5) * (utm + U.tm[i]);
             }
-            if (u[0] < P.tol_h)
-            {
-                u[3] = u[4] = u[5] = u[6] = u[7] = u[8] = T(0.0);
-            }
+            if (uh0 < tol_h) un0 = ut0 = unm = utm = T(0.0);
             else if (STAGE == 2)
-            {
-                const T ux = u[3] / u[0], uy = u[6] / u[0];
-                const T dtx = P.CFL * geo.dxl / (fabs(ux) + sqrt(P.g * u[0]));
-                const T dty = P.CFL * geo.dxl / (fabs(uy) + sqrt(P.g * u[0]));
-                leaf_dt = fmin(dtx, dty);
-            }
+                // (both directions give the same value but for their speeds: each lane its own)
+                leaf_dt = P.CFL * dxl / (fabs(un0 / uh0) + sqrt(g * uh0));
             if (STAGE == 2)
             {
-#pragma unroll
-                for (int k = 0; k < 9; ++k) lf.un[k][i] = u[k];
-                nan_seen |= (u[0] != u[0]);
-                mx.add(u, own.z[0]);
+                leaf_dt = fmin(leaf_dt, __shfl_xor_sync(pair, leaf_dt, 1));
+                // both lanes have read U^n mode 0 before lane 0 overwrites it
+                __syncwarp(pair);
+                put_un(uh0, un0, ut0, uhm, unm, utm);
+                nan_seen |= (uh0 != uh0);
+                if (!x) mx.add(uh0, ut0, z0);
             }
-            put_leaf(hout, a, u, own.z, wmark);
+            put(uh0, un0, ut0, uhm, unm, utm);
         }
-        else if (STAGE == 1) put_leaf(hout, a, pre, own.z, wmark);
+        else if (STAGE == 1) put(h0, n0, t0, pre_h, pre_n, pre_t);
         else
         {
-            T u[9];
-#pragma unroll
-            for (int k = 0; k < 9; ++k) u[k] = lf.un[k][i];
-            mx.add(u, own.z[0]);
-            put_leaf(hout, a, u, own.z, wmark);
+            const Axis<T> U = axis_of(lf, x);
+            const T uh = U.h0[i], un = U.n0[i], ut = U.t0[i];
+            if (!x) mx.add(uh, ut, z0);
+            put(uh, un, ut, U.hm[i], U.nm[i], U.tm[i]);
         }
-        if (STAGE == 2 && P.dt_leaf) P.dt_leaf[i] = leaf_dt;
+        if (!x && STAGE == 2 && P.dt_leaf) P.dt_leaf[i] = leaf_dt;
         dt_loc = fmin(dt_loc, leaf_dt);
     }
     if (!LIST)
@@ -762,7 +751,7 @@ __device__ __forceinline__ void k_mwdg2_stage_body(int bid, int nb, Leaves<T> lf
     }
 }
 template <typename T, int STAGE, bool LIST>
-__global__ void __launch_bounds__(kSolverThreads, sizeof(T) == 4 ? 5 : 2) k_mwdg2_stage(Leaves<T> lf, Hier<T> hin, Hier<T> hout, Scalars<T>* sc,
+__global__ void __launch_bounds__(kSolverThreads, kStageBlocks<T>) k_mwdg2_stage(Leaves<T> lf, Hier<T> hin, Hier<T> hout, Scalars<T>* sc,
                                                                 Params<T> P, const StepArgs<T>* args, bool friction,
                                                                 const int32_t* wet)
 {
@@ -842,7 +831,7 @@ __global__ void __launch_bounds__(kSolverThreads, sizeof(T) == 4 ? 6 : 3) k_hwfv
             const bool below_speed = (fabs(ux) < P.tol_s && fabs(uy) < P.tol_s);
             if (below_depth || below_speed) { own.qx[0] = T(0.0); own.qy[0] = T(0.0); }
             fric = !(below_depth || below_speed);
-            if (fric) friction_cell<T, false>(own, P, dt);
+            if (fric) friction_cell<T>(own, P, dt);
         }
         T nbh[4];
 #pragma unroll
@@ -866,7 +855,7 @@ __global__ void __launch_bounds__(kSolverThreads, sizeof(T) == 4 ? 6 : 3) k_hwfv
             Cell<T> c;
             if (nid[d] != -1) load_cell<T, false>(hr, nid[d], c);
             else { c.h[0] = gh[d]; c.qx[0] = gqx[d]; c.qy[0] = gqy[d]; c.z[0] = own.z[0]; }
-            if (fric) friction_cell<T, false>(c, P, dt);
+            if (fric) friction_cell<T>(c, P, dt);
             U[d] = V3<T>{c.h[0], c.qx[0], c.qy[0]};
             zn[d] = c.z[0];
         }
