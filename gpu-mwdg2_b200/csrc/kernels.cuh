@@ -42,6 +42,9 @@ template <typename T> struct Leaves
     // learned refinement proposal (null otherwise): same[i] = 1 where position i holds the
     // leaf it held in the last step (k_tile_emit), so un[i] already holds that leaf's state
     uint8_t* same;
+    // MWDG2 steps of one simulation (null otherwise): bit d set where neighbour d (N, E, S, W)
+    // is a significant parent, the leaf's neighbours there being finer (k_tile_emit)
+    uint8_t* par;
 };
 
 template <typename T> struct Scalars
@@ -54,6 +57,7 @@ template <typename T> struct Scalars
     unsigned long long enc, enc2, dec;   // parents encoded, re-encoded, and decoded in the bands
     uint32_t sig_level[16];           // significant parents decoded per level (levels above the bands)
     int32_t wet[2];                   // leaves not dry in RK stage 1 / stage 2 (wet-list lengths)
+    int32_t fix[2];                   // dry leaves whose state a stage changes (k_inplace_wet; list lengths)
     T next_max[4];                    // maxima of the state at the end of the step (eta, h, qx, z)
     T xs_factor;                      // 2^(M_BAR+1) of the extra-significance threshold (extra_eps)
     int32_t min_leaf;                 // lowest leaf level of this step's tree (k_tile_emit)
@@ -231,6 +235,7 @@ template <typename T> __device__ __forceinline__ void step_begin(Scalars<T>* sc,
     sc->dt_min = (sizeof(T) == 8) ? T(1.0e308) : T(3.0e38);
     sc->enc = 0; sc->enc2 = 0; sc->dec = 0;
     sc->wet[0] = 0; sc->wet[1] = 0;
+    sc->fix[0] = 0; sc->fix[1] = 0;
     sc->min_leaf = 1 << 30;
     // the expression of mra/extra_significance_kernel.cu, evaluated once per step instead of
     // once per parent (the same expression on the device gives the same bits everywhere)
@@ -372,12 +377,29 @@ template <typename T> __device__ __forceinline__ T extra_eps(T eps, int L, int l
 // parents. The scale-only kernels therefore skip parent levels below min_leaf, whose
 // values nothing would read; every output is the same bits.
 
+// One array's values of the four children at slot c for the scale re-encode between in-place RK
+// stages (INPL below; k_inplace_wet): leaves from the hierarchy (al), significant children,
+// whose flags are the bytes of cw, from the stage hierarchy (a).
+template <typename T> __device__ __forceinline__ void load_children(const T* a, const T* al, int c, uint32_t cw, T (&k)[4])
+{
+    load4(al + c, k);
+    if (cw & 0x01010101u)
+    {
+        T q[4];
+        load4(a + c, q);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if ((cw >> (8 * j)) & F_SIG) k[j] = q[j];
+    }
+}
+
 // Encode one parent (mra/encode_flow_kernel_{mw,hw}.cu), threshold it and OR in the
 // children's significance (mra/regularisation_kernel.cu). FULL = false re-encodes scale
 // coefficients of significant parents only (run_simulation.cu:573-588).
-template <typename T, bool MW, bool FULL, bool PM = false>
+// INPL, hl: load_children (scale-only).
+template <typename T, bool MW, bool FULL, bool PM = false, bool INPL = false>
 __device__ __forceinline__ void encode_parent(const Hier<T>& hr, const Scalars<T>* sc, int L, int level, int idx, T eps,
-                                              unsigned& n_done, const PropMask& pm = PropMask{})
+                                              unsigned& n_done, const PropMask& pm = PropMask{}, const Hier<T>& hl = Hier<T>{})
 {
     const int p = lvl_idx(level) + idx;
     // PM: a parent in a subtree the proposal leaves out keeps its flags and values
@@ -406,15 +428,22 @@ __device__ __forceinline__ void encode_parent(const Hier<T>& hr, const Scalars<T
             }
             mark = now | 1u;
         }
+        const uint32_t cw = INPL && level < L - 1 ? *reinterpret_cast<const uint32_t*>(hr.flags + c) : 0u;
 #pragma unroll
         for (int fld = 0; fld < 3; ++fld)
         {
             if (MW)
             {
                 T k[3][4];
-                load4(hr.s[fld][0] + c, k[0]); load4(hr.s[fld][1] + c, k[1]); load4(hr.s[fld][2] + c, k[2]);
+                if constexpr (INPL)
+                {
+#pragma unroll
+                    for (int m = 0; m < 3; ++m) load_children<T>(hr.s[fld][m], hl.s[fld][m], c, cw, k[m]);
+                }
+                else { load4(hr.s[fld][0] + c, k[0]); load4(hr.s[fld][1] + c, k[1]); load4(hr.s[fld][2] + c, k[2]); }
                 T s[3];
-                mw_encode_scale(k, s);
+                if constexpr (INPL) mw_encode_scale_stated(k, s);
+                else mw_encode_scale(k, s);
                 hr.s[fld][0][p] = s[0]; hr.s[fld][1][p] = s[1]; hr.s[fld][2][p] = s[2];
             }
             else
@@ -486,9 +515,9 @@ constexpr int kBandMaxLevel = 9;
 // (significant ones; FULL also clears the stale flag bits of the others, as k_level_sparse
 // does) before the parent itself: a child's data is touched by its parent's thread only,
 // and the sparse level needs no launch (and no scan of its flags) of its own.
-template <typename T, bool MW, bool FULL, bool FOLD = false, bool PM = false>
+template <typename T, bool MW, bool FULL, bool FOLD = false, bool PM = false, bool INPL = false>
 __device__ __forceinline__ void k_encode_level_body(Hier<T> hr, Scalars<T>* sc, int L, int level, T eps,
-                                                                         PropMask pm = PropMask{})
+                                                    PropMask pm = PropMask{}, Hier<T> hl = Hier<T>{})
 {
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     const bool in = idx < (1 << (2 * level));
@@ -518,7 +547,7 @@ __device__ __forceinline__ void k_encode_level_body(Hier<T> hr, Scalars<T>* sc, 
             lv = level;
             id = idx;
         }
-        if (go) encode_parent<T, MW, FULL, PM>(hr, sc, L, lv, id, eps, done, pm);
+        if (go) encode_parent<T, MW, FULL, PM, INPL>(hr, sc, L, lv, id, eps, done, pm, hl);
     }
     block_count(done, FULL ? &sc->enc : &sc->enc2);
 }
@@ -528,12 +557,21 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 4) k_encode_level(Hi
 {
     k_encode_level_body<T, MW, FULL, FOLD, PM>(hr, sc, L, level, eps, pm);
 }
+// The scale re-encode of stage hierarchy hs after an in-place stage 1 (load_children).
+template <typename T, bool FOLD>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 4) k_reencode_level(Hier<T> hs, Hier<T> hl, Scalars<T>* sc, int L, int level,
+                                                                           T eps)
+{
+    k_encode_level_body<T, true, false, FOLD, false, true>(hs, sc, L, level, eps, PropMask{}, hl);
+}
 
 // One field of one significant parent's encode: its scale coefficients (stored) and, for
 // FULL, the normalised maximum |detail| of that field (returned; 0 otherwise). The same
 // helper calls in the same order as one field of encode_parent.
-template <typename T, bool MW, bool FULL>
-__device__ __forceinline__ T encode_field(const Hier<T>& hr, const Scalars<T>* sc, int level, int idx, int fld)
+// INPL, hl: load_children (scale-only).
+template <typename T, bool MW, bool FULL, bool INPL = false>
+__device__ __forceinline__ T encode_field(const Hier<T>& hr, const Scalars<T>* sc, int level, int idx, int fld,
+                                          const Hier<T>& hl = Hier<T>{}, int L = 0)
 {
     const int p = lvl_idx(level) + idx;
     const int c = lvl_idx(level + 1) + 4 * idx;
@@ -545,9 +583,17 @@ __device__ __forceinline__ T encode_field(const Hier<T>& hr, const Scalars<T>* s
     if (MW)
     {
         T k[3][4];
-        load4(a0 + c, k[0]); load4(a1 + c, k[1]); load4(a2 + c, k[2]);
+        if constexpr (INPL)
+        {
+            const uint32_t cw = level < L - 1 ? *reinterpret_cast<const uint32_t*>(hr.flags + c) : 0u;
+            load_children<T>(a0, fld == 0 ? hl.s[0][0] : fld == 1 ? hl.s[1][0] : hl.s[2][0], c, cw, k[0]);
+            load_children<T>(a1, fld == 0 ? hl.s[0][1] : fld == 1 ? hl.s[1][1] : hl.s[2][1], c, cw, k[1]);
+            load_children<T>(a2, fld == 0 ? hl.s[0][2] : fld == 1 ? hl.s[1][2] : hl.s[2][2], c, cw, k[2]);
+        }
+        else { load4(a0 + c, k[0]); load4(a1 + c, k[1]); load4(a2 + c, k[2]); }
         T s[3];
-        mw_encode_scale(k, s);
+        if constexpr (INPL) mw_encode_scale_stated(k, s);
+        else mw_encode_scale(k, s);
         a0[p] = s[0]; a1[p] = s[1]; a2[p] = s[2];
         if (FULL)
         {
@@ -580,9 +626,9 @@ __device__ __forceinline__ T encode_field(const Hier<T>& hr, const Scalars<T>* s
 // waits on three dependent round trips, as a field's stores may alias the next one's
 // loads); the fields' detail norms meet in shared memory and are combined in field order,
 // as encode_parent combines them, before the flags.
-template <typename T, bool MW, bool FULL>
+template <typename T, bool MW, bool FULL, bool INPL = false>
 __device__ __forceinline__ void k_encode_band_body(Hier<T> hr, Scalars<T>* sc, int L, int lo, int depth, T eps,
-                                                     PropMask pm = PropMask{})
+                                                   PropMask pm = PropMask{}, Hier<T> hl = Hier<T>{})
 {
     if (!FULL && sc->min_leaf > lo + depth - 1) return;   // see scale_only_needed
     if (band_left_out(pm, lo)) return;
@@ -596,7 +642,7 @@ __device__ __forceinline__ void k_encode_band_body(Hier<T> hr, Scalars<T>* sc, i
         {
             const int fld = t >> sh, j = t & (n - 1);
             if (!(hr.flags[first + j] & F_SIG)) continue;
-            s_nd[fld][j] = encode_field<T, MW, FULL>(hr, sc, l, base + j, fld);
+            s_nd[fld][j] = encode_field<T, MW, FULL, INPL>(hr, sc, l, base + j, fld, hl, L);
         }
         __syncthreads();
         for (int j = threadIdx.x; j < n; j += blockDim.x)
@@ -632,6 +678,11 @@ __global__ void __launch_bounds__(256) k_encode_band(Hier<T> hr, Scalars<T>* sc,
                                                      PropMask pm = PropMask{})
 {
     k_encode_band_body<T, MW, FULL>(hr, sc, L, lo, depth, eps, pm);
+}
+template <typename T>
+__global__ void __launch_bounds__(256) k_reencode_band(Hier<T> hs, Hier<T> hl, Scalars<T>* sc, int L, int lo, int depth, T eps)
+{
+    k_encode_band_body<T, true, false, true>(hs, sc, L, lo, depth, eps, PropMask{}, hl);
 }
 
 // Decode one significant parent into its four children (mra/decoding_kernel_{mw,hw}.cu)
@@ -897,9 +948,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 4) k_decode_level(Hi
 // 4M threads. Op 0: FULL encode, 1: scale-only re-encode, 2: decode (values only, as
 // k_decode_level; keep: the keep-values decode of decode_parent, where only the parents
 // refined this step are listed and the encoded ones are just counted).
-template <typename T, bool MW, int OP, bool PM = false>
+template <typename T, bool MW, int OP, bool PM = false, bool INPL = false>
 __global__ void __launch_bounds__(256) k_level_sparse(Hier<T> hr, Scalars<T>* sc, int L, int level, T eps,
-                                                      PropMask pm = PropMask{}, bool keep = false)
+                                                      PropMask pm = PropMask{}, bool keep = false, Hier<T> hl = Hier<T>{})
 {
     if (OP == 1 && sc->min_leaf > level) return;   // see scale_only_needed
     __shared__ int list[8][256];   // per warp: up to 32 lanes x 8 parents
@@ -943,7 +994,7 @@ __global__ void __launch_bounds__(256) k_level_sparse(Hier<T> hr, Scalars<T>* sc
     {
         const int idx = list[warp][e];
         if (OP == 0) encode_parent<T, MW, true, PM>(hr, sc, L, level, idx, eps, done, pm);
-        else if (OP == 1) encode_parent<T, MW, false, PM>(hr, sc, L, level, idx, eps, done, pm);
+        else if (OP == 1) encode_parent<T, MW, false, PM, INPL>(hr, sc, L, level, idx, eps, done, pm, hl);
         else decode_parent<T, MW, false, PM>(hr, sc, L, level, idx, eps, done, pm);
     }
     if (OP == 0) block_count(done, &sc->enc);
@@ -1175,7 +1226,7 @@ __device__ __forceinline__ void put_act(const Leaves<T>& lf, int pos, int act, c
     lf.act[pos] = act;
 }
 
-template <typename T, bool NBL>
+template <typename T, bool NBL, bool PAR>
 __device__ __forceinline__ void emit_single_leaf(const Leaves<T>& lf, const uint8_t* flags, int L, int M, int xsz,
                                                  int ysz, int pos, int act, int l, const int32_t* n_prev)
 {
@@ -1185,6 +1236,11 @@ __device__ __forceinline__ void emit_single_leaf(const Leaves<T>& lf, const uint
     int32_t id;
     uint8_t lv;
     leaf_neighbour(flags, L, M, xsz, ysz, act, l, d, id, lv);
+    if (PAR)
+    {
+        const unsigned par = __ballot_sync(0xfu, id != -1 && lv < L && (flags[id] & F_SIG));
+        if (d == 0) lf.par[pos] = (uint8_t)par;
+    }
     lf.nb[d][pos] = id;
     if (NBL) lf.nbl[d][pos] = lv;
 }
@@ -1198,8 +1254,8 @@ __device__ __forceinline__ void emit_single_leaf(const Leaves<T>& lf, const uint
 // 100-108), -1 across the DEM or mesh border (neighbours/find_neighbours.cu:51-428).
 // Neighbouring cells are found by dilated-integer steps on the leaf's Morton code.
 // NBL: also write the neighbours' levels (lf.nbl), which level_of(id) gives wherever the id
-// is not -1 (-1: the leaf's own level).
-template <typename T, bool NBL>
+// is not -1 (-1: the leaf's own level). PAR: also mark the neighbours that are parents (lf.par).
+template <typename T, bool NBL, bool PAR>
 __device__ __forceinline__ void k_tile_emit_body(Leaves<T> lf, const uint8_t* flags, const int32_t* offsets,
                                                             int L, int M, int xsz, int ysz, int32_t* min_leaf,
                                                             const int32_t* n_prev)
@@ -1225,14 +1281,14 @@ __device__ __forceinline__ void k_tile_emit_body(Leaves<T> lf, const uint8_t* fl
         if ((tcode & ((1 << (2 * (Tl - k))) - 1)) == 0)
         {
             if (min_leaf && threadIdx.x == 0) atomicMin(min_leaf, k);
-            emit_single_leaf<T, NBL>(lf, flags, L, M, xsz, ysz, off, lvl_idx(k) + (tcode >> (2 * (Tl - k))), k, n_prev);
+            emit_single_leaf<T, NBL, PAR>(lf, flags, L, M, xsz, ysz, off, lvl_idx(k) + (tcode >> (2 * (Tl - k))), k, n_prev);
         }
         return;
     }
     if (k == Tl)
     {
         if (min_leaf && threadIdx.x == 0) atomicMin(min_leaf, Tl);
-        emit_single_leaf<T, NBL>(lf, flags, L, M, xsz, ysz, off, lvl_idx(Tl) + tcode, Tl, n_prev);
+        emit_single_leaf<T, NBL, PAR>(lf, flags, L, M, xsz, ysz, off, lvl_idx(Tl) + tcode, Tl, n_prev);
         return;
     }
     if (threadIdx.x < 85)
@@ -1342,6 +1398,7 @@ __device__ __forceinline__ void k_tile_emit_body(Leaves<T> lf, const uint8_t* fl
                                 Y0 == 0, X0 == 0};
         const unsigned tc[4] = {Xe | dil_add(Ye, 2u, kYBits), dil_add(Xe, 1u, kXBits) | Ye, X0 | dil_sub(Y0, 2u, kYBits),
                                 dil_sub(X0, 1u, kXBits) | Y0};
+        unsigned par = 0;
 #pragma unroll
         for (int d = 0; d < 4; ++d)
         {
@@ -1355,19 +1412,21 @@ __device__ __forceinline__ void k_tile_emit_body(Leaves<T> lf, const uint8_t* fl
                 else if (d == 0 || d == 2) lt = halo[d][t & lmask & kXBits];
                 else lt = halo[d][(t & lmask & kYBits) >> 1];
                 lv = lev < lt ? lev : lt;
+                if (PAR) par |= (lev < lt ? 1u : 0u) << d;
                 id = lvl_idx(lv) + (int)(t >> (2 * (L - lv)));
             }
             lf.nb[d][pos] = id;
             if (NBL) lf.nbl[d][pos] = (uint8_t)lv;
         }
+        if (PAR) lf.par[pos] = (uint8_t)par;
     }
 }
-template <typename T, bool NBL>
+template <typename T, bool NBL, bool PAR>
 __global__ void __launch_bounds__(kTileThreads, 8) k_tile_emit(Leaves<T> lf, const uint8_t* flags, const int32_t* offsets,
                                                             int L, int M, int xsz, int ysz, int32_t* min_leaf,
                                                             const int32_t* n_prev)
 {
-    k_tile_emit_body<T, NBL>(lf, flags, offsets, L, M, xsz, ysz, min_leaf, n_prev);
+    k_tile_emit_body<T, NBL, PAR>(lf, flags, offsets, L, M, xsz, ysz, min_leaf, n_prev);
 }
 
 // Initial leaf list: every finest cell, in Z order.

@@ -142,6 +142,25 @@ template <typename T> MW_HD void mw_encode_details(const T (&c)[3][4], T (&d)[3]
     d[0][2] = analyse<T, 1, 2>(c); d[1][2] = analyse<T, 2, 2>(c); d[2][2] = analyse<T, 3, 2>(c);
 }
 
+// mw_encode_scale with the sums' fused products stated. A compiler may fuse the first sum's
+// first or second product, and only row 1 (1x) has two that are not exact or zero: this is
+// what it does in the plain scale re-encode, whose bits the in-place one has to give.
+template <typename T, int r> MW_HD T analyse_scale(const T (&c)[3][4])
+{
+    T a = fma(tap<T, 0, 0, r, 0>(), c[0][0], tap<T, 0, 0, r, 1>() * c[1][0]);
+    a = fma(tap<T, 0, 0, r, 2>(), c[2][0], a);
+    a = fma(tap<T, 0, 1, r, 0>(), c[0][2], a); a = fma(tap<T, 0, 1, r, 1>(), c[1][2], a); a = fma(tap<T, 0, 1, r, 2>(), c[2][2], a);
+    a = fma(tap<T, 0, 2, r, 0>(), c[0][1], a); a = fma(tap<T, 0, 2, r, 1>(), c[1][1], a); a = fma(tap<T, 0, 2, r, 2>(), c[2][1], a);
+    a = fma(tap<T, 0, 3, r, 0>(), c[0][3], a); a = fma(tap<T, 0, 3, r, 1>(), c[1][3], a); a = fma(tap<T, 0, 3, r, 2>(), c[2][3], a);
+    return a / T(2.0);
+}
+template <typename T> MW_HD void mw_encode_scale_stated(const T (&c)[3][4], T (&s)[3])
+{
+    s[0] = analyse_scale<T, 0>(c);
+    s[1] = analyse_scale<T, 1>(c);
+    s[2] = analyse_scale<T, 2>(c);
+}
+
 // classes/SubDetail.h:12-46 -- max |detail| over one field's nine details
 template <typename T> MW_HD T mw_detail_max(const T (&d)[3][3])
 {

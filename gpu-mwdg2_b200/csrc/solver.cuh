@@ -262,9 +262,10 @@ __device__ __forceinline__ NbFace<T> neighbour(const Hier<T>& hr, const Axis<T>&
     }
     NbFace<T> r;
     r.h0 = h[0]; r.n0 = n[0]; r.t0 = t[0]; r.z0 = z[0];
-    // modes in the order 0, 1x, 1y, as the reference sums them
+    // modes in the order 0, 1x, 1y, as the reference sums them, both products fused (stated,
+    // since the selects may otherwise keep the compiler from it)
     const T bx = x ? bm : bt, by = x ? bt : bm;
-    auto at = [&](const T (&v)[3]) { return face(P3<T>{v[0], x ? v[1] : v[2], x ? v[2] : v[1]}, P3<T>{T(1.0), bx, by}); };
+    auto at = [&](const T (&v)[3]) { return fma(x ? v[2] : v[1], by, fma(x ? v[1] : v[2], bx, v[0])); };
     r.hf = at(h); r.nf = at(n); r.tf = at(t); r.zf = at(z);
     const T e[3] = {z[0] + h[0], z[1] + h[1], z[2] + h[2]};
     r.etaf = at(e);
@@ -509,6 +510,184 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 5) k_stage_dry(Leave
     k_stage_dry_body<T, STAGE>(blockIdx.x, gridDim.x, lf, hin, hout, sc, P, friction, dry, dry1, pm, clean_tag);
 }
 
+// ---------------------------------------------------------------- RK stages in place
+//
+// Steps whose two stages take the wet list (reference decode, no proposal): U* of a leaf stands
+// in the hierarchy itself. Almost every leaf is dry and ends both stages as it started, so
+// it is left alone: the wet test checks that the stage would put the same elevations back
+// (eta = (eta - z) + z), and with friction k_apply clears its mode-0 discharge, which the decode
+// left as rounding noise. The wet list's kernel, and the test for the few dry leaves that do
+// change, write their results to the leaf's slot of the stage hierarchy, and k_apply copies them
+// into the hierarchy once no leaf reads the old state any more. Neighbours that are significant parents (Leaves::par) take
+// their U* from the stage hierarchy, where the scale re-encode puts it.
+// Marks of stage 1 (`mark`): 0 wet, 1 dry and standing, 2 dry and changed. A standing leaf's
+// U^n is not stored: it is the hierarchy's own value (k_fill_un writes it where a getter needs it).
+// It replaces two writers of the dry leaves that moved 30 + 21 values a leaf. 4096^2 catchment,
+// 1 % wet, FP32 (ncu, per launch, stage 1 / 2): wet test 34 / 33 and dry writer 126 / 91 us
+// beside the wet list's kernel -> wet test 44 / 46, wet list 23 / 22, k_apply 19 / 6 us one after
+// another; step 0.637 -> 0.492 ms, FP64 (dry start) 0.911 -> 0.693 ms.
+
+// Position in a list of `n` entries for each lane with `in`, one atomic per warp.
+__device__ __forceinline__ int list_slot(bool in, int32_t* n)
+{
+    const unsigned mask = __ballot_sync(0xffffffffu, in);
+    const int lane = threadIdx.x & 31;
+    int base = 0;
+    if (mask)
+    {
+        if (lane == 0) base = atomicAdd(n, __popc(mask));
+        base = __shfl_sync(0xffffffffu, base, 0);
+    }
+    return base + __popc(mask & ((1u << lane) - 1u));
+}
+
+// Wet test of one in-place stage (the rule of k_stage_wet): wet leaves to `wet`, dry leaves
+// whose state changes to `fix`, their new values to their slots of hs.
+// Stage 1 (marks -> mark): U* = U^n with the depth after ghost cells and no discharge under
+// friction. Stage 2 (mark: stage 1's; marks -> mark2): U^{n+1} = U^n, which has to be put back
+// only where stage 1 moved the leaf; dry leaves enter the next step's maxima and report
+// initial_tstep as their CFL step.
+template <typename T, int STAGE>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 4) k_inplace_wet(Leaves<T> lf, Hier<T> hr, Hier<T> hs, Scalars<T>* sc, Params<T> P,
+                                                                        const StepArgs<T>* args, bool friction, uint8_t* mark,
+                                                                        uint8_t* mark2, int32_t* wet, int32_t* fix)
+{
+    const T dt = args->dt;
+    const Bnd<T>& B = args->B;
+    const int n = sc->n_leaves;
+    bool any_dry = false;
+    StateMax<T> mx;
+    for (int i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x)
+    {
+        const int i = i0 + threadIdx.x;
+        bool is_wet = false, is_fix = false;
+        if (i < n)
+        {
+            const int a = lf.act[i];
+            int32_t nid[4];
+#pragma unroll
+            for (int d = 0; d < 4; ++d) nid[d] = lf.nb[d][i];
+            const unsigned par = STAGE == 2 ? lf.par[i] : 0u;
+            const uint8_t m1 = STAGE == 2 ? mark[i] : 0;
+            const bool border = (nid[0] == -1) | (nid[1] == -1) | (nid[2] == -1) | (nid[3] == -1);
+            const int level = border ? lf.lvl[i] : 0;
+            const T e0 = hr.s[0][0][a], z0 = hr.s[3][0][a];
+            const T qx0 = border || (STAGE == 2 && !friction) ? hr.s[1][0][a] : T(0.0);
+            const T qy0 = border ? hr.s[2][0][a] : T(0.0);
+            T e1 = T(0.0), z1 = T(0.0), e2 = T(0.0), z2 = T(0.0);
+            if (STAGE == 1) { e1 = hr.s[0][1][a]; z1 = hr.s[3][1][a]; e2 = hr.s[0][2][a]; z2 = hr.s[3][2][a]; }
+            T nbh[4];
+#pragma unroll
+            for (int d = 0; d < 4; ++d)
+            {
+                const T* const eta = (par >> d) & 1u ? hs.s[0][0] : hr.s[0][0];
+                nbh[d] = (nid[d] != -1) ? eta[nid[d]] - hr.s[3][0][nid[d]] : T(0.0);
+            }
+            T h0 = e0 - z0;
+            T gh[4], gqx[4], gqy[4];
+            ghost_pass(h0, qx0, qy0, z0, nid, level, a, P, B, dt, gh, gqx, gqy);
+            bool is_dry = h0 < P.tol_h;
+#pragma unroll
+            for (int d = 0; d < 4; ++d) is_dry = is_dry && ((nid[d] != -1) ? nbh[d] : gh[d]) < P.tol_h;
+            is_wet = !is_dry;
+            any_dry |= is_dry;
+            T u[9];
+            if (STAGE == 1)
+            {
+                const T h1 = e1 - z1, h2 = e2 - z2;
+                const bool stands = h0 + z0 == e0 && h1 + z1 == e1 && h2 + z2 == e2;
+                is_fix = is_dry && !stands;
+                mark[i] = is_wet ? 0 : stands ? 1 : 2;
+                if (is_fix)
+                {
+                    u[0] = h0; u[1] = h1; u[2] = h2;
+                    u[3] = friction ? T(0.0) : hr.s[1][0][a];
+                    u[6] = friction ? T(0.0) : hr.s[2][0][a];
+#pragma unroll
+                    for (int m = 1; m < 3; ++m) { u[3 + m] = hr.s[1][m][a]; u[6 + m] = hr.s[2][m][a]; }
+#pragma unroll
+                    for (int k = 0; k < 9; ++k) lf.un[k][i] = u[k];
+                    const T z[3] = {z0, z1, z2};
+                    put_leaf(hs, a, u, z);
+                }
+            }
+            else
+            {
+                mark2[i] = is_dry ? 1 : 0;
+                is_fix = is_dry && m1 == 0;
+                if (is_dry)
+                {
+                    // U^n of a standing leaf is the hierarchy's own value
+                    if (m1 == 1) mx.add(e0 - z0, friction ? T(0.0) : qx0, z0);
+                    else mx.add(lf.un[0][i], lf.un[3][i], z0);
+                    if (P.dt_leaf) P.dt_leaf[i] = P.initial_tstep;
+                }
+                if (is_fix)
+                {
+                    const T z[3] = {z0, hr.s[3][1][a], hr.s[3][2][a]};
+#pragma unroll
+                    for (int k = 0; k < 9; ++k) u[k] = lf.un[k][i];
+                    put_leaf(hs, a, u, z);
+                }
+            }
+        }
+        int at = list_slot(is_wet, &sc->wet[STAGE - 1]);
+        if (is_wet) wet[at] = i;
+        at = list_slot(is_fix, &sc->fix[STAGE - 1]);
+        if (is_fix) fix[at] = i;
+    }
+    if (STAGE == 2)
+    {
+        mx.flush(sc);
+        if (__syncthreads_or(any_dry) && threadIdx.x == 0) atomic_min_nn(&sc->dt_min, P.initial_tstep);
+    }
+}
+
+// The listed leaves' results from their slots of the stage hierarchy into the hierarchy;
+// mark (stage 1 with friction): also the standing leaves' mode-0 discharge cleared.
+template <typename T>
+__global__ void __launch_bounds__(256) k_apply(Leaves<T> lf, Hier<T> hs, Hier<T> hr, const Scalars<T>* sc, int stage, const int32_t* wet,
+                                               const int32_t* fix, const uint8_t* mark)
+{
+    if (mark)
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < sc->n_leaves; i += gridDim.x * blockDim.x)
+        {
+            if (mark[i] != 1) continue;
+            const int a = lf.act[i];
+            hr.s[1][0][a] = T(0.0);
+            hr.s[2][0][a] = T(0.0);
+        }
+    const int nw = sc->wet[stage - 1], n = nw + sc->fix[stage - 1];
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
+    {
+        const int a = lf.act[k < nw ? wet[k] : fix[k - nw]];
+        T v[9];
+#pragma unroll
+        for (int j = 0; j < 9; ++j) v[j] = hs.s[j / 3][j % 3][a];
+#pragma unroll
+        for (int j = 0; j < 9; ++j) hr.s[j / 3][j % 3][a] = v[j];
+    }
+}
+
+// U^n (the leaf state) of the leaves that stood through both stages of an in-place step.
+template <typename T>
+__global__ void __launch_bounds__(256) k_fill_un(Leaves<T> lf, Hier<T> hr, const Scalars<T>* sc, const uint8_t* mark, const uint8_t* mark2)
+{
+    const int n = sc->n_leaves;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    {
+        if (mark[i] != 1 || !mark2[i]) continue;
+        const int a = lf.act[i];
+#pragma unroll
+        for (int m = 0; m < 3; ++m)
+        {
+            lf.un[m][i] = hr.s[0][m][a] - hr.s[3][m][a];
+            lf.un[3 + m][i] = hr.s[1][m][a];
+            lf.un[6 + m][i] = hr.s[2][m][a];
+        }
+    }
+}
+
 // Resident blocks of k_mwdg2_stage per SM that its registers are held to (64 in FP32, 128 in
 // FP64, with a few spills): 8 / 4 took 135.8 us for the dam-break step and 3.74 ms for the
 // ensemble's where 6 / 3 took 148.6 us and 3.94 ms; 9 / 5 and 10 / 6 are within noise of it.
@@ -532,10 +711,12 @@ template <typename T> constexpr int kStageBlocks = sizeof(T) == 4 ? 8 : 4;
 // list of the 2048^2 urban case FP32 86.2 / 58.5 -> 74.9 / 56.3 us; step of eight ensemble
 // members FP32 3.90 -> 3.52 ms. Four lanes per leaf (a face each) evaluated too much twice
 // (dam break step 142 -> 158 us, ensemble 4.37 -> 4.96 ms where this form takes 3.74).
-template <typename T, int STAGE, bool LIST>
+// INPL (stage 2 of an in-place step, mark: stage 1's marks): hin is the hierarchy, whose
+// significant parents' U* stands in hout, the stage hierarchy, which also takes the results.
+template <typename T, int STAGE, bool LIST, bool INPL = false>
 __device__ __forceinline__ void k_mwdg2_stage_body(int bid, int nb, Leaves<T> lf, Hier<T> hin, Hier<T> hout, Scalars<T>* sc,
                                                                 Params<T> P, const StepArgs<T>* args, bool friction,
-                                                                const int32_t* wet)
+                                                                const int32_t* wet, const uint8_t* mark = nullptr)
 {
     const T dt = args->dt;
     const Hier<T>& hr = hin;
@@ -643,9 +824,11 @@ __device__ __forceinline__ void k_mwdg2_stage_body(int bid, int nb, Leaves<T> lf
         const int code = a - lvl_idx(level);
         const T xc = cell_centre(compact(code), dxl), yc = cell_centre(compact(code >> 1), dxl);
         const bool in_extent = !((xc >= P.xsz * P.dx) || (yc >= P.ysz * P.dx));
-        const NbFace<T> H = neighbour(hr, A, x, true, id_hi, id_hi == -1 ? level : level_of(id_hi), gh_hi, gn_hi, gt_hi, z0, xc, yc,
+        const unsigned par = INPL ? lf.par[i] >> (x ? 1 : 0) : 0u;   // bits 0 and 2: the lane's faces
+        const bool p_hi = INPL && (par & 1u), p_lo = INPL && (par & 4u);
+        const NbFace<T> H = neighbour(p_hi ? hout : hr, p_hi ? axis_of(hout, x) : A, x, true, id_hi, id_hi == -1 ? level : level_of(id_hi), gh_hi, gn_hi, gt_hi, z0, xc, yc,
                                       dxl, STAGE == 1 && fric, P, dt);
-        const NbFace<T> W = neighbour(hr, A, x, false, id_lo, id_lo == -1 ? level : level_of(id_lo), gh_lo, gn_lo, gt_lo, z0, xc, yc,
+        const NbFace<T> W = neighbour(p_lo ? hout : hr, p_lo ? axis_of(hout, x) : A, x, false, id_lo, id_lo == -1 ? level : level_of(id_lo), gh_lo, gn_lo, gt_lo, z0, xc, yc,
                                       dxl, STAGE == 1 && fric, P, dt);
         // operators/copy_to_buf_assem_sol.cu: the stage-1 result of a leaf that is not
         // updated is its state before limiting
@@ -696,7 +879,13 @@ __device__ __forceinline__ void k_mwdg2_stage_body(int bid, int nb, Leaves<T> lf
             const T on = __shfl_xor_sync(pair, L0.qy, 1), ot = __shfl_xor_sync(pair, L0.qx, 1);
             T uh0 = h0 + dt * (L0.h + oh), un0 = n0 + dt * (L0.qx + on), ut0 = t0 + dt * (L0.qy + ot);
             T uhm = hm + dt * L1.h, unm = nm + dt * L1.qx, utm = tm + dt * L1.qy;
-            if (STAGE == 2)
+            if (STAGE == 2 && INPL && mark[i] == 1)
+            {
+                // a leaf that stood in stage 1: U^n is U*
+                uh0 = T(0.5) * (uh0 + (A.h0[a] - z0)); un0 = T(0.5) * (un0 + n0); ut0 = T(0.5) * (ut0 + t0);
+                uhm = T(0.5) * (uhm + pre_h); unm = T(0.5) * (unm + pre_n); utm = T(0.5) * (utm + pre_t);
+            }
+            else if (STAGE == 2)
             {
                 const Axis<T> U = axis_of(lf, x);
                 uh0 = T(0.5) * (uh0 + U.h0[i]); un0 = T(0.5) * (un0 + U.n0[i]); ut0 = T(0.5) * (ut0 + U.t0[i]);
@@ -718,6 +907,13 @@ __device__ __forceinline__ void k_mwdg2_stage_body(int bid, int nb, Leaves<T> lf
             put(uh0, un0, ut0, uhm, unm, utm);
         }
         else if (STAGE == 1) put(h0, n0, t0, pre_h, pre_n, pre_t);
+        else if (INPL && mark[i] == 1)
+        {
+            const T uh = A.h0[a] - z0;
+            put_un(uh, n0, t0, pre_h, pre_n, pre_t);
+            if (!x) mx.add(uh, t0, z0);
+            put(uh, n0, t0, pre_h, pre_n, pre_t);
+        }
         else
         {
             const Axis<T> U = axis_of(lf, x);
@@ -756,6 +952,14 @@ __global__ void __launch_bounds__(kSolverThreads, kStageBlocks<T>) k_mwdg2_stage
                                                                 const int32_t* wet)
 {
     k_mwdg2_stage_body<T, STAGE, LIST>(blockIdx.x, gridDim.x, lf, hin, hout, sc, P, args, friction, wet);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kSolverThreads, kStageBlocks<T>) k_inplace_stage2(Leaves<T> lf, Hier<T> hr, Hier<T> hs, Scalars<T>* sc,
+                                                                               Params<T> P, const StepArgs<T>* args, const int32_t* wet,
+                                                                               const uint8_t* mark)
+{
+    k_mwdg2_stage_body<T, 2, true, true>(blockIdx.x, gridDim.x, lf, hr, hs, sc, P, args, false, wet, mark);
 }
 
 // max |h0| of the stage-2 leaf state after ghost cells (run_simulation.cu:613-620).
@@ -935,7 +1139,8 @@ __global__ void __launch_bounds__(kSolverThreads, sizeof(T) == 4 ? 6 : 3) k_hwfv
 // covers the whole tile.
 template <typename T>
 __device__ __forceinline__ void k_sample_points_body(Leaves<T> lf, Hier<T> hr, Scalars<T>* sc, int L, const int32_t* codes, int np,
-                                const int32_t* tile_offsets, int ntiles, T* out)
+                                const int32_t* tile_offsets, int ntiles, T* out, const uint8_t* mark = nullptr,
+                                const uint8_t* mark2 = nullptr)
 {
     const int k = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (k >= np) return;   // the whole warp
@@ -964,17 +1169,20 @@ __device__ __forceinline__ void k_sample_points_body(Leaves<T> lf, Hier<T> hr, S
     if (lane != 0) return;
     const int a = lf.act[lo];
     const T z0 = hr.s[3][0][a];
-    const T eta = lf.un[0][lo] + z0;
+    // mark, mark2 (in-place steps): a leaf that stood through both stages has its state in hr
+    const bool stood = mark && mark[lo] == 1 && mark2[lo];
+    const T eta = stood ? hr.s[0][0][a] : lf.un[0][lo] + z0;
     out[4 * k + 0] = eta - z0;
-    out[4 * k + 1] = lf.un[3][lo];
-    out[4 * k + 2] = lf.un[6][lo];
+    out[4 * k + 1] = stood ? hr.s[1][0][a] : lf.un[3][lo];
+    out[4 * k + 2] = stood ? hr.s[2][0][a] : lf.un[6][lo];
     out[4 * k + 3] = z0;
 }
 template <typename T>
 __global__ void k_sample_points(Leaves<T> lf, Hier<T> hr, Scalars<T>* sc, int L, const int32_t* codes, int np,
-                                const int32_t* tile_offsets, int ntiles, T* out)
+                                const int32_t* tile_offsets, int ntiles, T* out, const uint8_t* mark = nullptr,
+                                const uint8_t* mark2 = nullptr)
 {
-    k_sample_points_body<T>(lf, hr, sc, L, codes, np, tile_offsets, ntiles, out);
+    k_sample_points_body<T>(lf, hr, sc, L, codes, np, tile_offsets, ntiles, out, mark, mark2);
 }
 
 // Leaf state with the bed coefficients gathered from the hierarchy, 12 rows of n values.
