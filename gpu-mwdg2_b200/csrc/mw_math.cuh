@@ -29,7 +29,10 @@ enum : uint8_t {
 // ---------------------------------------------------------------- indexing
 // utilities/get_lvl_idx.cuh:11-24 -- first slot of level n (3 padding slots)
 // (level <= 15: the library allows max_ref_lvl <= 14 and indexes levels up to L + 1)
-MW_HD int lvl_idx(int level) { return ((1 << (2 * level)) - 1) / 3 + 3; }
+// (4^n - 1) / 3 has every even bit below 2 n set: a mask instead of a division, which the leaf
+// topology would evaluate eight times per leaf (HWFV1 step of the 4096^2 catchment, 13.8 M
+// leaves: 0.692 -> 0.680 ms)
+MW_HD int lvl_idx(int level) { return (int)(0x55555555u & ((1u << (2 * level)) - 1u)) + 3; }
 
 // Level of a hierarchy index h >= 3 (inverse of lvl_idx): 3 (h - 3) + 1 lies in
 // [4^l, 4^(l+1)), so l is half the position of its highest set bit (32 bits hold it for
