@@ -595,7 +595,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 4) k_inplace_wet(Lea
             if (STAGE == 1)
             {
                 const T h1 = e1 - z1, h2 = e2 - z2;
-                const bool stands = h0 + z0 == e0 && h1 + z1 == e1 && h2 + z2 == e2;
+                // (a depth that a boundary segment reset has to be the hierarchy's own as well: the
+                // elevations alone may agree by rounding)
+                const bool stands = h0 == e0 - z0 && h0 + z0 == e0 && h1 + z1 == e1 && h2 + z2 == e2;
                 is_fix = is_dry && !stands;
                 mark[i] = is_wet ? 0 : stands ? 1 : 2;
                 if (is_fix)
