@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kTileThreads, 8) k_members_tile_emit(const __g
 {
     if (!on[blockIdx.y]) return;
     const MemberArgs<T>& a = tab.m[blockIdx.y];
-    k_tile_emit_body<T, false, true>(a.lf, a.hr.flags, a.tile_counts, L, a.M, a.xsz, a.ysz, &a.sc->min_leaf, &a.sc->n_prev);
+    k_tile_emit_body<T, false, false>(a.lf, a.hr.flags, a.tile_counts, L, a.M, a.xsz, a.ysz, &a.sc->min_leaf, &a.sc->n_prev);
 }
 
 // The member of this block of a per-leaf launch (one-dimensional grid) and the block's

@@ -42,8 +42,9 @@ template <typename T> struct Leaves
     // learned refinement proposal (null otherwise): same[i] = 1 where position i holds the
     // leaf it held in the last step (k_tile_emit), so un[i] already holds that leaf's state
     uint8_t* same;
-    // MWDG2 steps of one simulation (null otherwise): bit d set where neighbour d (N, E, S, W)
-    // is a significant parent, the leaf's neighbours there being finer (k_tile_emit)
+    // MWDG2 steps with RK stages in place (k_inplace_wet; not written for others): bit d set
+    // where neighbour d (N, E, S, W) is a significant parent, the leaf's neighbours there being
+    // finer (k_tile_emit)
     uint8_t* par;
 };
 

@@ -894,7 +894,10 @@ template <typename T> mwdg2_status Sim<T>::enqueue_device()
         ++launches_;
         mw::k_tile_scan<T><<<1, 1024, 0, st_>>>(tile_counts_, ntiles_, sc_);
         ++launches_;
-        const auto emit = mw ? mw::k_tile_emit<T, false, true> : mw::k_tile_emit<T, false, false>;
+        // the parent marks where this step's stages read them; without an epsilon only the first
+        // step has an emit, and a later one may run in place on its marks
+        const bool par = mw && (in_place() || !(eps > T(0)));
+        const auto emit = par ? mw::k_tile_emit<T, false, true> : mw::k_tile_emit<T, false, false>;
         emit<<<ntiles_, mw::kTileThreads, 0, st_>>>(lf_, hr_.flags, tile_counts_, L_, M_, cs_.xsz, cs_.ysz, &sc_->min_leaf,
                                                     &sc_->n_prev);
         ++launches_;

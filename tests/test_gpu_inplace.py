@@ -61,3 +61,33 @@ def test_in_place_stages_match_oracle(tmp_path, L, manning, limit, eps):
     finally:
         sim.close()
         orc.close()
+
+
+def test_in_place_stages_without_epsilon(tmp_path):
+    """With epsilon 0 only the first step builds the leaf list (every finest cell), before any step
+    can run in place; the later steps' in-place stages use its parent marks, also after steps of
+    the keep-values decode between them. Against the oracle as above."""
+    L, n = 7, 128
+    z = cases.fbm_surface(n, 0.8, 5, 29.37)
+    level = float(np.sort(z.ravel())[int(0.02 * z.size)])
+    c = cases.fbm_catchment(str(tmp_path), L=L, relief=29.37, seed=5, limitslopes=True, sim_time=600.0, t_peak=60.0,
+                            start_depth=np.maximum(0.0, np.round(level, 3) + 0.00037 - z))
+    sim, orc = mwdg2_b200.Simulation(c.par, precision=64, epsilon=0.0), oracle_py.Oracle(c.par, 64, epsilon=0.0)
+    try:
+        for s in range(1, 13):
+            if s in (1, 3, 6, 8):   # the keep-values decode in steps 1 to 2 and 6 to 7
+                sim.set_decode_mode("keep" if s in (1, 6) else "reference")
+                orc.set_keep_values(s in (1, 6))
+            ok, dt, nl = sim.step()
+            ok2, dt2, nl2 = orc.step()
+            assert ok and ok2 and nl == nl2 == n * n, f"step {s}: {nl} leaves, {nl2} in the oracle"
+            assert abs(dt - dt2) <= 1e-9 * dt2, f"step {s}: dt {dt}, {dt2} in the oracle"
+            if s % 2:
+                continue
+            assert_same_topology(sim.leaves(), orc.leaves(), f"step {s}")
+            a, b = sim.state(), orc.state()
+            for f in a:
+                assert rel_err(a[f], b[f]) <= 1e-10, f"step {s}: {f}"
+    finally:
+        sim.close()
+        orc.close()
