@@ -42,9 +42,9 @@ template <typename T> struct Leaves
     // learned refinement proposal (null otherwise): same[i] = 1 where position i holds the
     // leaf it held in the last step (k_tile_emit), so un[i] already holds that leaf's state
     uint8_t* same;
-    // MWDG2 steps with RK stages in place (k_inplace_wet; not written for others): bit d set
+    // MWDG2 steps with RK stages in place (k_inplace_wet; not written for others): bit 4 + d set
     // where neighbour d (N, E, S, W) is a significant parent, the leaf's neighbours there being
-    // finer (k_tile_emit)
+    // finer (k_tile_emit). The same bytes as the dry marks of stage 2, which take bit 0.
     uint8_t* par;
 };
 
@@ -1240,7 +1240,7 @@ __device__ __forceinline__ void emit_single_leaf(const Leaves<T>& lf, const uint
     if (PAR)
     {
         const unsigned par = __ballot_sync(0xfu, id != -1 && lv < L && (flags[id] & F_SIG));
-        if (d == 0) lf.par[pos] = (uint8_t)par;
+        if (d == 0) lf.par[pos] = (uint8_t)(par << 4);
     }
     lf.nb[d][pos] = id;
     if (NBL) lf.nbl[d][pos] = lv;
@@ -1419,7 +1419,7 @@ __device__ __forceinline__ void k_tile_emit_body(Leaves<T> lf, const uint8_t* fl
             lf.nb[d][pos] = id;
             if (NBL) lf.nbl[d][pos] = (uint8_t)lv;
         }
-        if (PAR) lf.par[pos] = (uint8_t)par;
+        if (PAR) lf.par[pos] = (uint8_t)(par << 4);
     }
 }
 template <typename T, bool NBL, bool PAR>

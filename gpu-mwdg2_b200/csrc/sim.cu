@@ -172,8 +172,9 @@ private:
     // bands of up to kBandDepth tree levels at and below level kBandMaxLevel, bottom first
     struct Band { int lo, depth, grid; };
     std::vector<Band> bands_;
-    int32_t* wet_list_ = nullptr;       // leaves that are not dry in an RK stage
-    int32_t* fix_list_ = nullptr;       // dry leaves that an in-place stage changes
+    // leaves that are not dry in an RK stage; from its end backwards, the dry leaves that an
+    // in-place stage changes
+    int32_t* wet_list_ = nullptr;
     bool un_lazy_ = false;              // the last step was in place: un of standing leaves is not stored
     mw::StepArgs<T>* d_args_ = nullptr; // this step's dt and boundary values (device)
     mw::StepArgs<T>* h_args_ = nullptr; // pinned; copied to d_args_ by the step's first operation
@@ -185,7 +186,7 @@ private:
     // kernel, so a step's launches do not depend on the leaf count and can be replayed.
     int grid_leaf_ = 0, grid_wet_ = 0, grid_dry_ = 0, grid_stage_ = 0, grid_inplace_ = 0;
     uint8_t* dry_ = nullptr;            // dry marks of RK stage 1 (k_stage_wet -> k_stage_dry)
-    uint8_t* dry2_ = nullptr;           // and of stage 2
+    uint8_t* dry2_ = nullptr;           // and of stage 2, which share their bytes with lf_.par
     // learned proposal and keep-values decode: per hierarchy index, the tag of the last step
     // in which the leaf there was dry in both stages (k_stage_wet<2>, on steps whose two
     // stages take the wet list)
@@ -314,14 +315,15 @@ private:
     }
     template <int STAGE> void inplace_stage(bool fric)
     {
+        int32_t* const fix = wet_list_ + F_ - 1;
         mw::k_inplace_wet<T, STAGE><<<grid_inplace_, 256, 0, st_>>>(lf_, hr_, hs_, sc_, P_, d_args_, fric, dry_, dry2_, wet_list_,
-                                                                    fix_list_);
+                                                                    fix);
         if (STAGE == 1)
             mw::k_mwdg2_stage<T, 1, true><<<grid_stage_, mw::kSolverThreads, 0, st_>>>(lf_, hr_, hs_, sc_, P_, d_args_, fric,
                                                                                        wet_list_);
         else
             mw::k_inplace_stage2<T><<<grid_stage_, mw::kSolverThreads, 0, st_>>>(lf_, hr_, hs_, sc_, P_, d_args_, wet_list_, dry_);
-        mw::k_apply<T><<<grid_leaf_, 256, 0, st_>>>(lf_, hs_, hr_, sc_, STAGE, wet_list_, fix_list_,
+        mw::k_apply<T><<<grid_leaf_, 256, 0, st_>>>(lf_, hs_, hr_, sc_, STAGE, wet_list_, fix,
                                                                 STAGE == 1 && fric ? dry_ : nullptr);
         launches_ += 3;
     }
@@ -571,10 +573,9 @@ template <typename T> mwdg2_status Sim<T>::init(const char* par, const mwdg2_opt
     if (mw_)
     {
         if (mwdg2_status s = dalloc(wet_list_, F_)) return s;
-        if (mwdg2_status s = dalloc(fix_list_, F_)) return s;
-        if (mwdg2_status s = dalloc(lf_.par, F_)) return s;
         if (mwdg2_status s = dalloc(dry_, F_)) return s;
         if (mwdg2_status s = dalloc(dry2_, F_)) return s;
+        lf_.par = dry2_;
         CU(cudaStreamCreateWithFlags(&st2_, cudaStreamNonBlocking));
         CU(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
         CU(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));

@@ -542,7 +542,8 @@ __device__ __forceinline__ int list_slot(bool in, int32_t* n)
 }
 
 // Wet test of one in-place stage (the rule of k_stage_wet): wet leaves to `wet`, dry leaves
-// whose state changes to `fix`, their new values to their slots of hs.
+// whose state changes to a second list that fills the same array from its end (`fix`, its last
+// entry, backwards: no leaf is in both), their new values to their slots of hs.
 // Stage 1 (marks -> mark): U* = U^n with the depth after ghost cells and no discharge under
 // friction. Stage 2 (mark: stage 1's; marks -> mark2): U^{n+1} = U^n, which has to be put back
 // only where stage 1 moved the leaf; dry leaves enter the next step's maxima and report
@@ -567,7 +568,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 4) k_inplace_wet(Lea
             int32_t nid[4];
 #pragma unroll
             for (int d = 0; d < 4; ++d) nid[d] = lf.nb[d][i];
-            const unsigned par = STAGE == 2 ? lf.par[i] : 0u;
+            const unsigned par = STAGE == 2 ? lf.par[i] >> 4 : 0u;
             const uint8_t m1 = STAGE == 2 ? mark[i] : 0;
             const bool border = (nid[0] == -1) | (nid[1] == -1) | (nid[2] == -1) | (nid[3] == -1);
             const int level = border ? lf.lvl[i] : 0;
@@ -615,7 +616,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 4) k_inplace_wet(Lea
             }
             else
             {
-                mark2[i] = is_dry ? 1 : 0;
+                mark2[i] = (uint8_t)(par << 4 | (is_dry ? 1u : 0u));   // (lf.par, for the wet list)
                 is_fix = is_dry && m1 == 0;
                 if (is_dry)
                 {
@@ -636,7 +637,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 4) k_inplace_wet(Lea
         int at = list_slot(is_wet, &sc->wet[STAGE - 1]);
         if (is_wet) wet[at] = i;
         at = list_slot(is_fix, &sc->fix[STAGE - 1]);
-        if (is_fix) fix[at] = i;
+        if (is_fix) fix[-at] = i;
     }
     if (STAGE == 2)
     {
@@ -662,7 +663,7 @@ __global__ void __launch_bounds__(256) k_apply(Leaves<T> lf, Hier<T> hs, Hier<T>
     const int nw = sc->wet[stage - 1], n = nw + sc->fix[stage - 1];
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
     {
-        const int a = lf.act[k < nw ? wet[k] : fix[k - nw]];
+        const int a = lf.act[k < nw ? wet[k] : fix[nw - k]];
         T v[9];
 #pragma unroll
         for (int j = 0; j < 9; ++j) v[j] = hs.s[j / 3][j % 3][a];
@@ -678,7 +679,7 @@ __global__ void __launch_bounds__(256) k_fill_un(Leaves<T> lf, Hier<T> hr, const
     const int n = sc->n_leaves;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     {
-        if (mark[i] != 1 || !mark2[i]) continue;
+        if (mark[i] != 1 || !(mark2[i] & 1)) continue;
         const int a = lf.act[i];
 #pragma unroll
         for (int m = 0; m < 3; ++m)
@@ -826,7 +827,7 @@ __device__ __forceinline__ void k_mwdg2_stage_body(int bid, int nb, Leaves<T> lf
         const int code = a - lvl_idx(level);
         const T xc = cell_centre(compact(code), dxl), yc = cell_centre(compact(code >> 1), dxl);
         const bool in_extent = !((xc >= P.xsz * P.dx) || (yc >= P.ysz * P.dx));
-        const unsigned par = INPL ? lf.par[i] >> (x ? 1 : 0) : 0u;   // bits 0 and 2: the lane's faces
+        const unsigned par = INPL ? lf.par[i] >> (x ? 5 : 4) : 0u;   // bits 0 and 2: the lane's faces
         const bool p_hi = INPL && (par & 1u), p_lo = INPL && (par & 4u);
         const NbFace<T> H = neighbour(p_hi ? hout : hr, p_hi ? axis_of(hout, x) : A, x, true, id_hi, id_hi == -1 ? level : level_of(id_hi), gh_hi, gn_hi, gt_hi, z0, xc, yc,
                                       dxl, STAGE == 1 && fric, P, dt);
@@ -1172,7 +1173,7 @@ __device__ __forceinline__ void k_sample_points_body(Leaves<T> lf, Hier<T> hr, S
     const int a = lf.act[lo];
     const T z0 = hr.s[3][0][a];
     // mark, mark2 (in-place steps): a leaf that stood through both stages has its state in hr
-    const bool stood = mark && mark[lo] == 1 && mark2[lo];
+    const bool stood = mark && mark[lo] == 1 && (mark2[lo] & 1);
     const T eta = stood ? hr.s[0][0][a] : lf.un[0][lo] + z0;
     out[4 * k + 0] = eta - z0;
     out[4 * k + 1] = stood ? hr.s[1][0][a] : lf.un[3][lo];

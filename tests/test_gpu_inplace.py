@@ -91,3 +91,29 @@ def test_in_place_stages_without_epsilon(tmp_path):
     finally:
         sim.close()
         orc.close()
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+def test_in_place_stages_take_no_memory_of_their_own(tmp_path, precision):
+    """What an MWDG2 simulation holds on the device, as its arrays' sizes give it: two hierarchies
+    (12 and 9 coefficient arrays), the flags, and per finest cell the leaf list (25 bytes with the
+    four neighbour ids and the wet list), two dry marks and nine state values. The in-place
+    stages use these arrays only. cudaMalloc hands out large arrays in units of 2 MiB; 12 MiB are
+    left for everything small (streams, events, scalars), where one more index per finest cell
+    would take 18."""
+    import torch
+
+    L, unit = 11, 2 << 20
+    F, n_det, P = 4 ** L, (4 ** L - 1) // 3 + 3, precision // 8
+    n_all = n_det + F
+    arrays = 21 * [n_all * P] + 9 * [F * P] + 6 * [4 * F] + 3 * [F] + [n_det]
+    want = sum(-(-(a + 64) // unit) * unit for a in arrays)
+    warm = cases.fbm_catchment(str(tmp_path / "small"), L=7)
+    c = cases.fbm_catchment(str(tmp_path / "case"), L=L)
+    mwdg2_b200.Simulation(warm.par, precision=precision).close()   # the context and the modules
+    before = torch.cuda.mem_get_info()[0]
+    sim = mwdg2_b200.Simulation(c.par, precision=precision)
+    held = before - torch.cuda.mem_get_info()[0]
+    sim.close()
+    print(f"held {held}, arrays {want}, rest {held - want}")
+    assert held - want <= 12 << 20, f"{held - want} bytes beyond the arrays"
