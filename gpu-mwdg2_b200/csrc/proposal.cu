@@ -75,14 +75,15 @@ cudaError_t set_smem_attrs()
     return e;
 }
 
-// Host samples (FP32 features [n][113..128]) -> device BF16 rows of 128.
-mwdg2_status upload_features(DevBufs& b, const float* feats, int nfeat, int64_t n, __nv_bfloat16*& d)
+// Host samples (FP32 features [n][113..128]) -> device BF16 rows of 128, on the stream of the
+// kernels that read them (the copy from pageable memory returns before it is done).
+mwdg2_status upload_features(DevBufs& b, const float* feats, int nfeat, int64_t n, __nv_bfloat16*& d, cudaStream_t st)
 {
     std::vector<uint16_t> h((size_t)n * mlp::kIn, 0);
     for (int64_t i = 0; i < n; ++i)
         for (int k = 0; k < nfeat && k < mlp::kIn; ++k) h[(size_t)i * mlp::kIn + k] = to_bf16(feats[(size_t)i * nfeat + k]);
     CUDA_OK(b.alloc(d, h.size()));
-    CUDA_OK(cudaMemcpy(d, h.data(), h.size() * 2, cudaMemcpyHostToDevice));
+    CUDA_OK(cudaMemcpyAsync(d, h.data(), h.size() * 2, cudaMemcpyHostToDevice, st));
     return MWDG2_OK;
 }
 
@@ -124,7 +125,7 @@ mwdg2_status mwdg2_mlp_forward(const float* params, const float* feats, int nfea
     __nv_bfloat16* d_feat = nullptr;
     CUDA_OK(b.alloc(d_prm, mlp::kParams));
     CUDA_OK(cudaMemcpy(d_prm, params, sizeof(float) * mlp::kParams, cudaMemcpyHostToDevice));
-    if (mwdg2_status s = upload_features(b, feats, nfeat, n, d_feat)) return s;
+    if (mwdg2_status s = upload_features(b, feats, nfeat, n, d_feat, nullptr)) return s;
     CUDA_OK(b.alloc(d_log, (size_t)n * mlp::kOut));
     CUDA_OK(b.alloc(d_prop, (size_t)n * mlp::kOut));
     CUDA_OK(b.alloc(d_err, 1));
@@ -155,7 +156,7 @@ mwdg2_status mwdg2_mlp_grad(const float* params, const float* feats, int nfeat, 
     __nv_bfloat16* d_feat = nullptr;
     CUDA_OK(b.alloc(d_prm, mlp::kParams));
     CUDA_OK(cudaMemcpy(d_prm, params, sizeof(float) * mlp::kParams, cudaMemcpyHostToDevice));
-    if (mwdg2_status s = upload_features(b, feats, nfeat, n, d_feat)) return s;
+    if (mwdg2_status s = upload_features(b, feats, nfeat, n, d_feat, nullptr)) return s;
     CUDA_OK(b.alloc(d_lab, (size_t)n));
     CUDA_OK(cudaMemcpy(d_lab, labels, (size_t)n, cudaMemcpyHostToDevice));
     CUDA_OK(b.alloc(d_grad, mlp::kParams));
@@ -190,11 +191,11 @@ mwdg2_status mwdg2_trainer_create(const float* init_params, float lr, int device
     if (e == cudaSuccess) e = cudaMalloc(&t->loss, sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&t->err, sizeof(int));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&t->st, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMemcpy(t->prm, init_params, sizeof(float) * mlp::kParams, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(t->grad, 0, sizeof(float) * mlp::kParams);
-    if (e == cudaSuccess) e = cudaMemset(t->m, 0, sizeof(float) * mlp::kParams);
-    if (e == cudaSuccess) e = cudaMemset(t->v, 0, sizeof(float) * mlp::kParams);
-    if (e == cudaSuccess) e = cudaMemset(t->err, 0, sizeof(int));
+    if (e == cudaSuccess) e = cudaMemcpyAsync(t->prm, init_params, sizeof(float) * mlp::kParams, cudaMemcpyHostToDevice, t->st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(t->grad, 0, sizeof(float) * mlp::kParams, t->st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(t->m, 0, sizeof(float) * mlp::kParams, t->st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(t->v, 0, sizeof(float) * mlp::kParams, t->st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(t->err, 0, sizeof(int), t->st);
     if (e == cudaSuccess) e = set_smem_attrs();
     if (e != cudaSuccess)
     {
@@ -235,9 +236,9 @@ mwdg2_status mwdg2_trainer_step(mwdg2_trainer* t, const float* feats, int nfeat,
     DevBufs b;
     __nv_bfloat16* d_feat = nullptr;
     uint8_t* d_lab = nullptr;
-    if (mwdg2_status s = upload_features(b, feats, nfeat, n, d_feat)) return s;
+    if (mwdg2_status s = upload_features(b, feats, nfeat, n, d_feat, t->st)) return s;
     CUDA_OK(b.alloc(d_lab, (size_t)n));
-    CUDA_OK(cudaMemcpy(d_lab, labels, (size_t)n, cudaMemcpyHostToDevice));
+    CUDA_OK(cudaMemcpyAsync(d_lab, labels, (size_t)n, cudaMemcpyHostToDevice, t->st));
     return trainer_step_device(t, d_feat, d_lab, n, pos_weight, loss_out);
 }
 

@@ -157,6 +157,8 @@ private:
     int n_leaves_ = 0;
     int solver_blocks_ = 0, red_blocks_ = 0;
     int device_ = 0;
+    // every upload, set and kernel of this simulation is on its own stream: the legacy stream does
+    // not order with a non-blocking one, and a copy from pageable memory returns before it is done
     cudaStream_t st_ = nullptr;
     std::vector<void*> allocs_;
     mw::Hier<T> hr_{};
@@ -538,7 +540,7 @@ template <typename T> mwdg2_status Sim<T>::init(const char* par, const mwdg2_opt
     hs_.flags = hr_.flags;
     // HWFV1: the second buffer starts at zero (only slots that a step writes are ever read)
     if (!mw_)
-        for (int f = 0; f < 3; ++f) CU(cudaMemset(hs_.s[f][0], 0, sizeof(T) * (size_t)n_all_));
+        for (int f = 0; f < 3; ++f) CU(cudaMemsetAsync(hs_.s[f][0], 0, sizeof(T) * (size_t)n_all_, st_));
     // leaves (capacity: every finest cell)
     if (mwdg2_status s = dalloc(lf_.act, F_)) return s;
     if (mwdg2_status s = dalloc(lf_.lvl, F_)) return s;
@@ -561,7 +563,7 @@ template <typename T> mwdg2_status Sim<T>::init(const char* par, const mwdg2_opt
     {
         char* block = nullptr;
         if (mwdg2_status s = dalloc(block, scal_bytes_)) return s;
-        CU(cudaMemset(block, 0, scal_bytes_));
+        CU(cudaMemsetAsync(block, 0, scal_bytes_, st_));
         sc_ = reinterpret_cast<mw::Scalars<T>*>(block);
         if (nst > 0) d_stage_out_ = reinterpret_cast<T*>(block + stage_off);
         char* hblock = nullptr;
@@ -627,7 +629,8 @@ template <typename T> mwdg2_status Sim<T>::init(const char* par, const mwdg2_opt
         CU(cudaMalloc(&d_raster, sizeof(T) * 4 * F_));
         for (int f = 0; f < 4; ++f)
         {
-            cudaError_t e = cudaMemcpy(d_raster + (size_t)f * F_, cs_.raster[f].data(), sizeof(T) * F_, cudaMemcpyHostToDevice);
+            cudaError_t e = cudaMemcpyAsync(d_raster + (size_t)f * F_, cs_.raster[f].data(), sizeof(T) * F_,
+                                            cudaMemcpyHostToDevice, st_);
             if (e != cudaSuccess) { cudaFree(d_raster); CU(e); }
             std::vector<T>().swap(cs_.raster[f]);
         }
@@ -651,7 +654,7 @@ template <typename T> mwdg2_status Sim<T>::init(const char* par, const mwdg2_opt
     {
         std::vector<uint8_t> fl(n_det_);
         for (int i = 0; i < n_det_; ++i) fl[i] = mw::F_SIG | (cs_.preflag[i] ? mw::F_PRE : 0);
-        CU(cudaMemcpy(hr_.flags, fl.data(), n_det_, cudaMemcpyHostToDevice));
+        CU(cudaMemcpyAsync(hr_.flags, fl.data(), n_det_, cudaMemcpyHostToDevice, st_));
     }
 
     P_.L = L_; P_.M = M_; P_.xsz = cs_.xsz; P_.ysz = cs_.ysz; P_.limit = cs_.limitslopes ? 1 : 0;
@@ -678,13 +681,12 @@ template <typename T> mwdg2_status Sim<T>::init(const char* par, const mwdg2_opt
         else mw::k_topo_level<T, false><<<nb, 256, 0, st_>>>(hr_, sc_, L_, level, cs_.epsilon);
     }
     CU(cudaGetLastError());
-    CU(cudaStreamSynchronize(st_));
     {
-        int32_t nl = (int32_t)F_;
-        CU(cudaMemcpy(&sc_->n_leaves, &nl, sizeof(nl), cudaMemcpyHostToDevice));
-        int32_t zero = 0;
-        CU(cudaMemcpy(&sc_->status, &zero, sizeof(zero), cudaMemcpyHostToDevice));
+        const int32_t nl = (int32_t)F_;
+        CU(cudaMemcpyAsync(&sc_->n_leaves, &nl, sizeof(nl), cudaMemcpyHostToDevice, st_));
+        CU(cudaMemsetAsync(&sc_->status, 0, sizeof(sc_->status), st_));
     }
+    CU(cudaStreamSynchronize(st_));
     if (mwdg2_status st = set_timing(o.verbose >= 2 ? 2 : 0)) return st;
     t_start_ = std::chrono::steady_clock::now();
     return MWDG2_OK;
@@ -1115,12 +1117,12 @@ template <typename T> mwdg2_status Sim<T>::freeze_alloc()
     if (!lf_.same)
     {
         if (mwdg2_status s = dalloc(lf_.same, F_)) return s;
-        CU(cudaMemset(lf_.same, 0, F_));
+        CU(cudaMemsetAsync(lf_.same, 0, F_, st_));
     }
     if (!clean_tag_)
     {
         if (mwdg2_status s = dalloc(clean_tag_, n_all_)) return s;
-        CU(cudaMemset(clean_tag_, 0, sizeof(uint32_t) * (size_t)n_all_));
+        CU(cudaMemsetAsync(clean_tag_, 0, sizeof(uint32_t) * (size_t)n_all_, st_));
     }
     return MWDG2_OK;
 }
@@ -1136,26 +1138,26 @@ template <typename T> mwdg2_status Sim<T>::prop_alloc()
     if (mwdg2_status s = dalloc(d_lab_, (size_t)prop_nC_)) return s;
     const size_t nring = (size_t)std::max<int64_t>(1, prop_nC_ / mw::kPropTile);
     if (mwdg2_status s = dalloc(d_ring_, nring)) return s;
-    CU(cudaMemset(d_ring_, 0xff, nring * sizeof(uint16_t)));   // every tile runs until labels exist
+    CU(cudaMemsetAsync(d_ring_, 0xff, nring * sizeof(uint16_t), st_));   // every tile runs until labels exist
     {
         std::vector<int32_t> nodes;
         for (const auto& src : cs_.srcs) nodes.push_back(src.code >> (2 * (L_ - (prop_C_ + 1))));
         if (mwdg2_status s = dalloc(d_prop_src_, std::max<size_t>(1, nodes.size()))) return s;
         if (!nodes.empty())
-            CU(cudaMemcpy(d_prop_src_, nodes.data(), sizeof(int32_t) * nodes.size(), cudaMemcpyHostToDevice));
+            CU(cudaMemcpyAsync(d_prop_src_, nodes.data(), sizeof(int32_t) * nodes.size(), cudaMemcpyHostToDevice, st_));
     }
     if (mwdg2_status s = freeze_alloc()) return s;
     if (mwdg2_status s = dalloc(d_act_, (size_t)prop_nC_ * 4)) return s;
     if (mwdg2_status s = dalloc(d_prop_, (size_t)prop_nC_ * 4)) return s;
     if (mwdg2_status s = dalloc(d_sig5_, (size_t)prop_nC_ * 4)) return s;
-    CU(cudaMemset(d_sig5_, 0, (size_t)prop_nC_ * 4));
+    CU(cudaMemsetAsync(d_sig5_, 0, (size_t)prop_nC_ * 4, st_));
     if (mwdg2_status s = dalloc(d_mlp_, mlp::kParams)) return s;
     if (mwdg2_status s = dalloc(d_mlp_pack_, mlp::kPackBytes)) return s;
     if (mwdg2_status s = dalloc(d_mlp_err_, 1)) return s;
-    CU(cudaMemset(d_lab_, 0, (size_t)prop_nC_));
-    CU(cudaMemset(d_act_, 0, (size_t)prop_nC_ * 4));
-    CU(cudaMemset(d_prop_, 1, (size_t)prop_nC_ * 4));
-    CU(cudaMemset(d_mlp_err_, 0, sizeof(int)));
+    CU(cudaMemsetAsync(d_lab_, 0, (size_t)prop_nC_, st_));
+    CU(cudaMemsetAsync(d_act_, 0, (size_t)prop_nC_ * 4, st_));
+    CU(cudaMemsetAsync(d_prop_, 1, (size_t)prop_nC_ * 4, st_));
+    CU(cudaMemsetAsync(d_mlp_err_, 0, sizeof(int), st_));
     CU(cudaFuncSetAttribute(mlp::k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)(mlp::FwdSmem::Total + 1024)));
     CU(cudaFuncSetAttribute(mw::k_mlp_propose<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1185,7 +1187,7 @@ mwdg2_status Sim<T>::proposal_enable(const float* params, int judge_every, float
         return proposal_record(prop_rec_);
     }
     if (mwdg2_status s = prop_alloc()) return s;
-    CU(cudaMemcpy(d_mlp_, params, sizeof(float) * mlp::kParams, cudaMemcpyHostToDevice));
+    CU(cudaMemcpyAsync(d_mlp_, params, sizeof(float) * mlp::kParams, cudaMemcpyHostToDevice, st_));
     mlp::k_mlp_pack<<<1, mlp::kRows, 0, st_>>>(d_mlp_, d_mlp_pack_);
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(st_));
@@ -1711,7 +1713,7 @@ template <typename T> mwdg2_status Sim<T>::decode_mode(int mode)
         std::vector<uint8_t> mask((size_t)n, 0);
         for (const auto& src : cs_.srcs) mask[(size_t)(src.code >> (2 * (L_ - (C + 1))))] = 1;
         if (mwdg2_status s = dalloc(d_keep_prop_, (size_t)n)) return s;
-        CU(cudaMemcpy(d_keep_prop_, mask.data(), (size_t)n, cudaMemcpyHostToDevice));
+        CU(cudaMemcpyAsync(d_keep_prop_, mask.data(), (size_t)n, cudaMemcpyHostToDevice, st_));
         prop_C_ = C;
         if (mwdg2_status s = dalloc(hs_tag_, n_all_)) return s;
     }
