@@ -217,15 +217,11 @@ template <typename T> MW_HD void hw_decode(T u, T a, T b, T g, T (&c)[4])
 
 // ---------------------------------------------------------------- flow algebra
 template <typename T> struct V3 { T h, qx, qy; };            // classes/FlowVector.h
-template <typename T> struct P3 { T _0, _1x, _1y; };          // classes/PlanarCoefficients.h
 
 template <typename T> MW_HD V3<T> operator+(const V3<T>& a, const V3<T>& b) { return {a.h + b.h, a.qx + b.qx, a.qy + b.qy}; }
 template <typename T> MW_HD V3<T> operator-(const V3<T>& a, const V3<T>& b) { return {a.h - b.h, a.qx - b.qx, a.qy - b.qy}; }
 template <typename T> MW_HD V3<T> operator*(T s, const V3<T>& a) { return {s * a.h, s * a.qx, s * a.qy}; }
 template <typename T> MW_HD V3<T> operator/(const V3<T>& a, T s) { return {a.h / s, a.qx / s, a.qy / s}; }
-
-// operators/eval_loc_face_val_dg2.cuh:7-15
-template <typename T> MW_HD T face(const P3<T>& s, const P3<T>& b) { return s._0 * b._0 + s._1x * b._1x + s._1y * b._1y; }
 
 // classes/FlowVector.h:13-48 (get_speed, calc_h_star, get_star)
 template <typename T> MW_HD V3<T> star(const V3<T>& U, T z, T z_inter, T tol_h)

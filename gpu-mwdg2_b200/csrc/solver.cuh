@@ -1,7 +1,7 @@
-// Per-leaf solver kernels: one thread per leaf, grid-stride over the device-side leaf
-// count. Each kernel gathers the leaf and its four neighbours straight from the
-// hierarchy and keeps all per-neighbour work in registers, replacing the reference's
-// sequence load_soln_and_nghbr_coeffs -> add_ghost_cells -> friction_implicit ->
+// Per-leaf solver kernels, grid-stride over the device-side leaf count: one thread per leaf, in
+// the DG2 stage kernels two lanes per leaf (one axis each). Each kernel gathers the leaf and
+// its neighbours straight from the hierarchy, replacing the reference's sequence
+// load_soln_and_nghbr_coeffs -> add_ghost_cells -> friction_implicit ->
 // copy_to_buf_assem_sol -> limit_slopes -> dg2_update (or fv1_update) -> get_dt_CFL
 // and its five materialised neighbour copies.
 #pragma once
@@ -10,22 +10,19 @@
 
 namespace mw {
 
-template <typename T> struct Cell { T h[3], qx[3], qy[3], z[3]; };
-
-// neighbours/load_soln_and_nghbr_coeffs.cu:3-104 (h = eta - z)
-template <typename T, bool MW> __device__ __forceinline__ void load_cell(const Hier<T>& hr, int a, Cell<T>& c)
+// A first-order cell (neighbours/load_soln_and_nghbr_coeffs.cu:3-104, h = eta - z). The loop over
+// the one mode changes the compiler's order of the loads: written out, k_hwfv1<float> spills more
+// (4096^2 catchment, two steps 1356 -> 1386 us).
+template <typename T> struct Cell { T h[1], qx[1], qy[1], z[1]; };
+template <typename T> __device__ __forceinline__ void load_cell(const Hier<T>& hr, int a, Cell<T>& c)
 {
 #pragma unroll
-    for (int m = 0; m < (MW ? 3 : 1); ++m)
+    for (int m = 0; m < 1; ++m)
     {
         c.z[m] = hr.s[3][m][a];
         c.h[m] = hr.s[0][m][a] - c.z[m];
         c.qx[m] = hr.s[1][m][a];
         c.qy[m] = hr.s[2][m][a];
-    }
-    if (!MW)
-    {
-        c.h[1] = c.h[2] = c.qx[1] = c.qx[2] = c.qy[1] = c.qy[2] = c.z[1] = c.z[2] = T(0.0);
     }
 }
 
@@ -137,8 +134,9 @@ __device__ __forceinline__ void ghost_pass(T& own_h0, T own_qx0, T own_qy0, T ow
 // operators/friction_implicit.cu:155-264 -- implicit friction on the mode-0 value and,
 // for MWDG2, on the four Gauss-point values, whose differences rebuild the slopes.
 // One out-of-line copy of the implicit Manning update of a point value (apply_friction):
-// the stage kernel applies it at up to 7 points per lane and would otherwise hold as many
-// inlined copies of its pow and divisions, which stall warps on instruction fetch.
+// the stage kernel applies it at 9 to 13 points per lane of a moving leaf (3 of the leaf, 3 of
+// each neighbour, 5 of one of another size) and would otherwise hold as many inlined copies
+// of its pow and divisions, which stall warps on instruction fetch.
 template <typename T> struct Q2 { T qx, qy; };
 template <typename T> __device__ __noinline__ Q2<T> friction_point(T h, T qx, T qy, T tol_h, T tol_s, T n, T g, T dt)
 {
@@ -150,17 +148,6 @@ template <typename T> __device__ __noinline__ Q2<T> friction_point(T h, T qx, T 
 template <typename T> __device__ __forceinline__ void friction_cell(Cell<T>& c, const Params<T>& P, T dt)
 {
     apply_friction(c.h[0], P.tol_h, P.tol_s, c.qx[0], c.qy[0], P.manning, P.g, dt);
-}
-
-// Friction of a DG2 cell's slopes along one axis: the point values at its two face centres
-// there (value -/+ slope), whose difference is the new slope.
-template <typename T>
-__device__ __forceinline__ void friction_slope(T h0, T qx0, T qy0, T hm, T& qxm, T& qym, const Params<T>& P, T dt)
-{
-    const Q2<T> lo = friction_point(h0 - hm, qx0 - qxm, qy0 - qym, P.tol_h, P.tol_s, P.manning, P.g, dt);
-    const Q2<T> hi = friction_point(h0 + hm, qx0 + qxm, qy0 + qym, P.tol_h, P.tol_s, P.manning, P.g, dt);
-    qxm = T(0.5) * (hi.qx - lo.qx);
-    qym = T(0.5) * (hi.qy - lo.qy);
 }
 
 // ---------------------------------------------------------------- DG2: two lanes per leaf
@@ -337,7 +324,8 @@ __device__ __forceinline__ void put_leaf_fv1(const Hier<T>& hout, int a, T h, T 
     mx.add(h, qx, z);
 }
 
-// Wet test of one RK stage (the rule of leaf_is_dry, after ghost cells): wet leaves are
+// Wet test of one RK stage: a leaf is dry when its own depth and its four neighbours' (after
+// ghost cells) are all below tol_h, and is then not updated, limited or rubbed. Wet leaves are
 // appended to `wet` (warp-aggregated) for k_mwdg2_stage<.., LIST=true> (a NaN depth is not
 // below tol_h, so a NaN leaf is listed and the stage kernel reports it), dry ones marked in
 // `dry` for k_stage_dry, which then runs beside the wet-list kernel (the two touch disjoint
@@ -692,7 +680,9 @@ __global__ void __launch_bounds__(256) k_fill_un(Leaves<T> lf, Hier<T> hr, const
 }
 
 // Resident blocks of k_mwdg2_stage per SM that its registers are held to (64 in FP32, 128 in
-// FP64, with a few spills): 8 / 4 took 135.8 us for the dam-break step and 3.74 ms for the
+// FP64). Bytes of spill stores / loads by ptxas: FP32 stage 1 144 / 76, stage 2 112 / 108, stage 2
+// in place 300 / 236 (each neighbour comes from one of two hierarchies); FP64 148 / 112, 96 / 120
+// and 152 / 156. 8 / 4 blocks took 135.8 us for the dam-break step and 3.74 ms for the
 // ensemble's where 6 / 3 took 148.6 us and 3.94 ms; 9 / 5 and 10 / 6 are within noise of it.
 template <typename T> constexpr int kStageBlocks = sizeof(T) == 4 ? 8 : 4;
 
@@ -707,8 +697,9 @@ template <typename T> constexpr int kStageBlocks = sizeof(T) == 4 ? 8 : 4;
 //
 // What bounds it: few wet leaves, one leaf's serial latency; many, instruction issue (IEEE
 // divisions, square roots and pow of the friction and the fluxes). Two lanes per leaf halve the
-// chain of a leaf without evaluating anything twice but its mean friction point and its own
-// mode-0 loads, and need about half the registers of a thread that holds all four faces.
+// chain of a leaf's faces, and need about half the registers of a thread that holds all four. What
+// concerns the leaf as a whole both lanes evaluate: its mean friction point, the speed test's
+// divisions, the cell's centre, the mode-0 update, sqrt(g h), the ghost cells of a border leaf.
 // Against one thread per leaf (ncu, per launch, stage 1 / 2): 256^2 dam break FP64, every leaf
 // wet, 33.3 / 33.7 -> 15.3 / 17.6 us; 1000 x 700 flood FP64 54.8 / 28.8 -> 34.5 / 23.1 us; wet
 // list of the 2048^2 urban case FP32 86.2 / 58.5 -> 74.9 / 56.3 us; step of eight ensemble
@@ -1023,7 +1014,7 @@ __global__ void __launch_bounds__(kSolverThreads, sizeof(T) == 4 ? 6 : 3) k_hwfv
 #pragma unroll
         for (int d = 0; d < 4; ++d) nid[d] = lf.nb[d][i];
         Cell<T> own;
-        load_cell<T, false>(hr, a, own);
+        load_cell(hr, a, own);
         // a NaN depth anywhere in the state (a NaN leaf with NaN neighbours is never updated)
         nan_seen |= (own.h[0] != own.h[0]);
         T gh[4], gqx[4], gqy[4];
@@ -1060,7 +1051,7 @@ __global__ void __launch_bounds__(kSolverThreads, sizeof(T) == 4 ? 6 : 3) k_hwfv
         for (int d = 0; d < 4; ++d)
         {
             Cell<T> c;
-            if (nid[d] != -1) load_cell<T, false>(hr, nid[d], c);
+            if (nid[d] != -1) load_cell(hr, nid[d], c);
             else { c.h[0] = gh[d]; c.qx[0] = gqx[d]; c.qy[0] = gqy[d]; c.z[0] = own.z[0]; }
             if (fric) friction_cell<T>(c, P, dt);
             U[d] = V3<T>{c.h[0], c.qx[0], c.qy[0]};
