@@ -250,7 +250,7 @@ private:
     cudaEvent_t ev_[9] = {};
     cudaEvent_t ev_step_[2] = {};
     double last_ms_[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    int64_t last_cnt_[11] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+    int64_t last_cnt_[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     int launches_ = 0;
     // learned refinement proposal (csrc/proposal_sim.cuh): record features and activity labels
     // (prop_rec_), propose the subtrees the encode and decode visit (prop_learned_); every
@@ -999,6 +999,7 @@ template <typename T> mwdg2_status Sim<T>::collect_step()
     last_cnt_[8] = (int64_t)(sizeof(mw::StepArgs<T>) + sizeof(mw::Src<T>) * cs_.srcs.size());
     last_cnt_[9] = (int64_t)scal_bytes_;
     last_cnt_[10] = mw ? (int64_t)sc_host_->prop_frozen : 0;
+    last_cnt_[11] = un_lazy_ ? 1 : 0;   // as the step's launch left it
     return MWDG2_OK;
 }
 
@@ -1732,7 +1733,7 @@ template <typename T> mwdg2_status Sim<T>::decode_mode(int mode)
 
 template <typename T> mwdg2_status Sim<T>::counters(int64_t* out, int n)
 {
-    for (int i = 0; i < n && i < 11; ++i) out[i] = last_cnt_[i];
+    for (int i = 0; i < n && i < 12; ++i) out[i] = last_cnt_[i];
     return MWDG2_OK;
 }
 

@@ -135,7 +135,8 @@ mwdg2_status mwdg2_set_timing(mwdg2_sim* sim, int mode);
  * step, [6] / [7] MWDG2 leaves not dry in RK stage 1 / stage 2 (0 for HWFV1), [8] bytes the
  * step copied host->device (dt, boundary and point-source values), [9] bytes it copied
  * device->host (its scalars and the stage-point values), [10] dry leaves that the RK stages
- * left as they stood (keep-values decode or learned proposal; MWDG2). n <= 11. */
+ * left as they stood (keep-values decode or learned proposal; MWDG2), [11] 1 where the RK
+ * stages ran in place (reference decode without a proposal, few wet leaves; MWDG2). n <= 12. */
 mwdg2_status mwdg2_last_step_counters(mwdg2_sim* sim, int64_t* out, int n);
 
 /* Water volume of the current state, sum over leaves of h0 x leaf area (m^3), reduced on

@@ -20,8 +20,8 @@ pytestmark = pytest.mark.gpu
 
 
 # (11, 0.0, True, 1e-3) is left out: at its step 6 a limiter decision sits on its threshold and
-# the CUDA path and the oracle part by 1.6e-8, in place or with every leaf written (the two
-# routes give the same bits there)
+# the CUDA path and the oracle part by 1.6e-8, in place or with every leaf written
+# (test_gpu_inplace_routes.py holds the two routes to each other there)
 @pytest.mark.parametrize("L,manning,limit,eps", [(7, 0.0, True, 1e-3), (8, 0.03, True, 1e-3), (9, 0.03, False, 1e-2),
                                                  (11, 0.03, False, 1e-3)])
 def test_in_place_stages_match_oracle(tmp_path, L, manning, limit, eps):
@@ -36,12 +36,14 @@ def test_in_place_stages_match_oracle(tmp_path, L, manning, limit, eps):
             if s in (8, 10):   # the keep-values decode for two steps
                 sim.set_decode_mode("keep" if s == 8 else "reference")
                 orc.set_keep_values(s == 8)
-            in_place += 10 * wet < leaves and s not in (8, 9)   # the rule, from the step before
+            expected = 10 * wet < leaves and s not in (8, 9)   # the rule, from the step before
             ok, dt, n = sim.step()
             ok2, dt2, n2 = orc.step()
             assert ok and ok2 and n == n2, f"step {s}: {n} leaves, {n2} in the oracle"
             assert abs(dt - dt2) <= 1e-9 * dt2, f"step {s}: dt {dt}, {dt2} in the oracle"
             k = sim.last_step_counters()
+            assert k["in_place"] == expected, f"step {s}: in place {k['in_place']}"
+            in_place += k["in_place"]
             wet, leaves = max(k["wet_stage1"], k["wet_stage2"]), k["leaves"]
             if s % 3 != 0:
                 continue       # two steps between reads of the state
@@ -84,6 +86,7 @@ def test_in_place_stages_without_epsilon(tmp_path):
             assert abs(dt - dt2) <= 1e-9 * dt2, f"step {s}: dt {dt}, {dt2} in the oracle"
             if s % 2:
                 continue
+            assert sim.last_step_counters()["in_place"] == (s not in (2, 6)), f"step {s}"
             assert_same_topology(sim.leaves(), orc.leaves(), f"step {s}")
             a, b = sim.state(), orc.state()
             for f in a:

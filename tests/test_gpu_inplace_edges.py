@@ -50,8 +50,8 @@ def test_segments_that_reset_dry_leaves(tmp_path, precision, manning):
             ok, dt, n = sim.step()
             _, dts, leaves = b.step()
             assert ok and dt == dts[0] and n == leaves[0], f"step {s}"
-            k = sim.last_step_counters()
-            assert 10 * max(k["wet_stage1"], k["wet_stage2"]) < k["leaves"], f"step {s}: too wet to run in place"
+            assert sim.last_step_counters()["in_place"] == (s > 1), f"step {s}"
+            assert b.member(0).last_step_counters()["in_place"] == 0, f"step {s}"
             if s % 3:
                 continue       # two steps between reads of the state
             m = b.member(0)
