@@ -308,8 +308,16 @@ private:
     // proposal. The keep-values decode and the proposal have their own frozen dry leaves, which
     // the dry-leaf writers of stage() leave alone as well, with tags that the scale re-encode
     // uses. Only where under a tenth of the leaves were wet: the wet list's kernel, which the
-    // writers run beside, is a launch of its own here (2048^2 urban case, 12-17 % wet, FP32:
-    // 0.520 ms a step with the writers, 0.530 in place; catchments of 1 % wet 0.637 and 0.492).
+    // writers run beside, is a launch of its own here, and it is what grows. Step in us with the
+    // writers / in place, the two taking turns on the same steps, by share of wet leaves:
+    //   catchment 4096^2 FP32  1 % 640 / 490, 7 % 749 / 625, 11 % 818 / 733, 20 % 957 / 941
+    //             4096^2 FP64  7 % 1227 / 1033, 14 % 1563 / 1453
+    //             2048^2 FP32  8 % 395 / 366, 13 % 426 / 404, 19 % 461 / 455
+    //             2048^2 FP64  8 % 605 / 564, 13 % 677 / 674, 16 % 723 / 735
+    //             1024^2 FP64  7 % 340 / 319, 13 % 379 / 378; 512^2 FP64  3-10 % 155-158 / 156-159
+    //   urban     4096^2 FP32 19 % 1768 / 1629, 2048^2 13 % 454 / 432, 1024^2 16 % 183 / 193
+    // Up to a tenth neither size, precision nor case loses more than noise; above it in place
+    // still wins on large cases and loses up to 5 % on small ones.
     bool in_place() const
     {
         auto few = [&](int stage) { return use_list(stage) && 10 * wet_prev_[stage - 1] < n_leaves_; };
