@@ -176,16 +176,17 @@ class Clocks:
                 "reasons": reasons, "samples": len(self.rows), "source": "nvml"}
 
 
-# DRAM bytes per leaf (dram__bytes_read.sum + dram__bytes_write.sum of the phase's kernels,
-# summed, divided by the step's leaves) from a one-pass ncu launch list of this workload
-# (4096^2, FP32, 3.0 M leaves). Keyed by (solver, P, timing phase).
-TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the phase's kernels (one kernel, three "
+TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the phase's kernels (one kernel, two "
                   "launches per capture) on the 2048^2 catchment (max_ref_lvl 11, 1.21 M leaves), per leaf, "
                   "x this run's leaves")
 PHASE_STEPS = 5
 REF_CPU_STEPS = 20   # the reference arm's timed steps on the host cores (at most)
-# DRAM bytes per leaf of the RK stages (phase 4: stage 1, phase 6: stage 2) in FP32
-TRAFFIC_B_PER_LEAF: dict = {("mwdg2", 4, 4): 181.0, ("mwdg2", 4, 6): 141.6}
+# DRAM bytes per leaf (dram__bytes_read.sum + dram__bytes_write.sum of the phase's kernels, summed,
+# divided by the step's leaves) in FP32 by (solver, P, timing phase, decode): leaf topology (3; its
+# writes stay in L2), RK stage 1 (4) and stage 2 (6). profiles/dram_stage_kernels_fbm2048_fp32.md.
+TRAFFIC_B_PER_LEAF: dict = {("mwdg2", 4, 3, "reference"): 2.4, ("mwdg2", 4, 4, "reference"): 79.7,
+                            ("mwdg2", 4, 6, "reference"): 42.0, ("mwdg2", 4, 3, "keep"): 2.4,
+                            ("mwdg2", 4, 4, "keep"): 128.2, ("mwdg2", 4, 6, "keep"): 62.7}
 
 
 def max_over_ranks(x: float, dist, device: str) -> float:
@@ -747,16 +748,17 @@ def main():
     # ids + 9P written + 9P of U^n = 30P + 16; stage 2: 21P + 16 (together the N(51P + 32)
     # solver term of the step formula below). HWFV1: 4P own + 16 B ids + 3P written.
     cand = {"leaf topology (k_tile_count + k_tile_scan + k_tile_emit)": (3, 40),
-            "RK stage 1 (k_stage_wet<1>, then k_stage_dry<1> beside k_mwdg2_stage<1> over the wet list; or "
-            "one k_mwdg2_stage<1> sweep)": (4, 30 * P + 16),
-            "RK stage 2 (k_stage_wet<2>, then k_stage_dry<2> beside k_mwdg2_stage<2> over the wet list; or "
-            "one k_mwdg2_stage<2> sweep)": (6, 21 * P + 16)}
+            "RK stage 1 (in place k_inplace_wet<1>, k_mwdg2_stage<1> over the wet list, k_apply; or k_stage_wet<1>, "
+            "then k_stage_dry<1> beside the list; or one sweep)": (4, 30 * P + 16),
+            "RK stage 2 (in place k_inplace_wet<2>, k_inplace_stage2, k_apply; or k_stage_wet<2>, then k_stage_dry<2> "
+            "beside k_mwdg2_stage<2> over the wet list; or one sweep)": (6, 21 * P + 16)}
     if a.solver == "hwfv1":
         cand = {"leaf topology (k_tile_count + k_tile_scan + k_tile_emit)": (3, 40),
                 "k_hwfv1 (gather, friction, FV1 update, CFL)": (4, 7 * P + 16)}
     kname, (kph, per_leaf) = max(cand.items(), key=lambda kv: mean_ph[kv[1][0]])
     kms = float(mean_ph[kph])
-    traffic = TRAFFIC_B_PER_LEAF.get((a.solver, P, kph)) if (a.workload, a.level) == ("catchment", 12) else None
+    traffic = (TRAFFIC_B_PER_LEAF.get((a.solver, P, kph, a.decode)) if (a.workload, a.level) == ("catchment", 12)
+               else None)
     achieved = per_leaf * n_mean_ph / (kms / 1e3) / 1e9
     # Algorithmic bytes per step of the reference-layout model, from each step's device
     # counters: E parents encoded, E2 re-encoded (scale only), D decoded, T detail slots,

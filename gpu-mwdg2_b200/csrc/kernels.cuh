@@ -195,8 +195,8 @@ __device__ __forceinline__ void block_max_atomic(T (&v)[N], T* const (&dst)[N])
 }
 
 // Sum of `v` over the block, called by every thread of it (valid in the first warp).
-// The per-level kernels count their parents with it. One atomic per warp on one address bound
-// them, since atomics on one address retire one after another (about 0.8 ns each, 2 x 131072
+// The level and band kernels count their parents with it. One atomic per warp on one address bound
+// the level kernels, since atomics on one address retire one after another (about 0.8 ns each, 2 x 131072
 // of them in a dense level-11 decode). Per block instead, and without a second counter that
 // the host can sum, on the 4096^2 catchment in FP32 (ncu, per launch): HWFV1 decode of levels
 // 10 and 11 132 -> 44 us, encode 89 -> 39 us; MWDG2 level 10 decode 82 -> 49 us, encode
