@@ -76,7 +76,8 @@ cudaError_t set_smem_attrs()
 }
 
 // Host samples (FP32 features [n][113..128]) -> device BF16 rows of 128, on the stream of the
-// kernels that read them (the copy from pageable memory returns before it is done).
+// kernels that read them (a copy from pageable memory may return before it is done: the stream is
+// waited for before the rows' host copy goes).
 mwdg2_status upload_features(DevBufs& b, const float* feats, int nfeat, int64_t n, __nv_bfloat16*& d, cudaStream_t st)
 {
     std::vector<uint16_t> h((size_t)n * mlp::kIn, 0);
@@ -84,6 +85,7 @@ mwdg2_status upload_features(DevBufs& b, const float* feats, int nfeat, int64_t 
         for (int k = 0; k < nfeat && k < mlp::kIn; ++k) h[(size_t)i * mlp::kIn + k] = to_bf16(feats[(size_t)i * nfeat + k]);
     CUDA_OK(b.alloc(d, h.size()));
     CUDA_OK(cudaMemcpyAsync(d, h.data(), h.size() * 2, cudaMemcpyHostToDevice, st));
+    CUDA_OK(cudaStreamSynchronize(st));
     return MWDG2_OK;
 }
 
@@ -196,6 +198,7 @@ mwdg2_status mwdg2_trainer_create(const float* init_params, float lr, int device
     if (e == cudaSuccess) e = cudaMemsetAsync(t->m, 0, sizeof(float) * mlp::kParams, t->st);
     if (e == cudaSuccess) e = cudaMemsetAsync(t->v, 0, sizeof(float) * mlp::kParams, t->st);
     if (e == cudaSuccess) e = cudaMemsetAsync(t->err, 0, sizeof(int), t->st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(t->st);   // the caller's parameters are read
     if (e == cudaSuccess) e = set_smem_attrs();
     if (e != cudaSuccess)
     {

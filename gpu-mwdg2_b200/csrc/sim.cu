@@ -158,7 +158,8 @@ private:
     int solver_blocks_ = 0, red_blocks_ = 0;
     int device_ = 0;
     // every upload, set and kernel of this simulation is on its own stream: the legacy stream does
-    // not order with a non-blocking one, and a copy from pageable memory returns before it is done
+    // not order with a non-blocking one, and a copy from pageable memory may return before it is
+    // done (so the stream is waited for before such a source goes)
     cudaStream_t st_ = nullptr;
     std::vector<void*> allocs_;
     mw::Hier<T> hr_{};
@@ -640,7 +641,6 @@ template <typename T> mwdg2_status Sim<T>::init(const char* par, const mwdg2_opt
             cudaError_t e = cudaMemcpyAsync(d_raster + (size_t)f * F_, cs_.raster[f].data(), sizeof(T) * F_,
                                             cudaMemcpyHostToDevice, st_);
             if (e != cudaSuccess) { cudaFree(d_raster); CU(e); }
-            std::vector<T>().swap(cs_.raster[f]);
         }
         const int grid = grid_for(F_, 256, 1 << 20);
         if (mw_) mw::k_init_finest<T, true><<<grid, 256, 0, st_>>>(d_raster, M_, cs_.xsz, cs_.ysz, hr_, lf_, fin);
@@ -655,6 +655,7 @@ template <typename T> mwdg2_status Sim<T>::init(const char* par, const mwdg2_opt
         }
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
+        for (int f = 0; f < 4; ++f) std::vector<T>().swap(cs_.raster[f]);   // read by their copies until here
         cudaFree(d_raster);
         CU(e);
     }
@@ -663,6 +664,7 @@ template <typename T> mwdg2_status Sim<T>::init(const char* par, const mwdg2_opt
         std::vector<uint8_t> fl(n_det_);
         for (int i = 0; i < n_det_; ++i) fl[i] = mw::F_SIG | (cs_.preflag[i] ? mw::F_PRE : 0);
         CU(cudaMemcpyAsync(hr_.flags, fl.data(), n_det_, cudaMemcpyHostToDevice, st_));
+        CU(cudaStreamSynchronize(st_));
     }
 
     P_.L = L_; P_.M = M_; P_.xsz = cs_.xsz; P_.ysz = cs_.ysz; P_.limit = cs_.limitslopes ? 1 : 0;
@@ -689,11 +691,9 @@ template <typename T> mwdg2_status Sim<T>::init(const char* par, const mwdg2_opt
         else mw::k_topo_level<T, false><<<nb, 256, 0, st_>>>(hr_, sc_, L_, level, cs_.epsilon);
     }
     CU(cudaGetLastError());
-    {
-        const int32_t nl = (int32_t)F_;
-        CU(cudaMemcpyAsync(&sc_->n_leaves, &nl, sizeof(nl), cudaMemcpyHostToDevice, st_));
-        CU(cudaMemsetAsync(&sc_->status, 0, sizeof(sc_->status), st_));
-    }
+    const int32_t nl = (int32_t)F_;
+    CU(cudaMemcpyAsync(&sc_->n_leaves, &nl, sizeof(nl), cudaMemcpyHostToDevice, st_));
+    CU(cudaMemsetAsync(&sc_->status, 0, sizeof(sc_->status), st_));
     CU(cudaStreamSynchronize(st_));
     if (mwdg2_status st = set_timing(o.verbose >= 2 ? 2 : 0)) return st;
     t_start_ = std::chrono::steady_clock::now();
@@ -1153,7 +1153,10 @@ template <typename T> mwdg2_status Sim<T>::prop_alloc()
         for (const auto& src : cs_.srcs) nodes.push_back(src.code >> (2 * (L_ - (prop_C_ + 1))));
         if (mwdg2_status s = dalloc(d_prop_src_, std::max<size_t>(1, nodes.size()))) return s;
         if (!nodes.empty())
+        {
             CU(cudaMemcpyAsync(d_prop_src_, nodes.data(), sizeof(int32_t) * nodes.size(), cudaMemcpyHostToDevice, st_));
+            CU(cudaStreamSynchronize(st_));
+        }
     }
     if (mwdg2_status s = freeze_alloc()) return s;
     if (mwdg2_status s = dalloc(d_act_, (size_t)prop_nC_ * 4)) return s;
@@ -1723,6 +1726,7 @@ template <typename T> mwdg2_status Sim<T>::decode_mode(int mode)
         for (const auto& src : cs_.srcs) mask[(size_t)(src.code >> (2 * (L_ - (C + 1))))] = 1;
         if (mwdg2_status s = dalloc(d_keep_prop_, (size_t)n)) return s;
         CU(cudaMemcpyAsync(d_keep_prop_, mask.data(), (size_t)n, cudaMemcpyHostToDevice, st_));
+        CU(cudaStreamSynchronize(st_));
         prop_C_ = C;
         if (mwdg2_status s = dalloc(hs_tag_, n_all_)) return s;
     }
